@@ -2,7 +2,8 @@
 amr2d_mhd that drives it (in-tree, amr2d_mhd_gb300/_build/).
 
 Every translation unit compiles in parallel with nvcc for sm_103a only.  Every
-translation unit but the FP32 stage kernels (stage_f32_*.cu) is compiled with
+translation unit but the FP32 stage and face kernels (stage_f32_*.cu,
+faces_f32_*.cu) is compiled with
 -fmad=false and the host code with -ffp-contract=off: that path reproduces the reference's
 floating-point operations one by one, so nothing may be fused.  The FP32 stage
 kernels (the FP32 bulk path's reconstruction, Riemann fluxes and RK update)
@@ -44,7 +45,7 @@ def _flags(src: str):
               "-I" + CSRC]
     if src.endswith(".cpp"):
         return ["-x", "cu"] + ARCH + common
-    fmad = ["-prec-div=false", "-prec-sqrt=false"] if src.startswith("stage_f32") else ["-fmad=false"]
+    fmad = ["-prec-div=false", "-prec-sqrt=false"] if src.startswith(("stage_f32", "faces_f32")) else ["-fmad=false"]
     return ARCH + common + fmad
 
 

@@ -231,9 +231,10 @@ __device__ __forceinline__ FaceJac muscl_face_jac(int lim, double wm, double w0,
   const double E = 1.0E-15;
   const double dA = w0 - wm, dB = w1 - w0, dC = w2 - w1;
   FaceJac J;
+  Native<double> m;
   double d;
   // left = w0 + phi(dB / (dA + E)) dA / 2
-  double phi = limiter_d(lim, limiter_ratio<double>(lim, dB, dA + E), d);
+  double phi = limiter_d(lim, limiter_ratio<double>(m, lim, dB, dA + E), d);
   J.left = w0 + 0.5 * phi * dA;
   double ldA = 0.5 * phi, ldB = 0.0;
   if (d != 0.0) {
@@ -245,7 +246,7 @@ __device__ __forceinline__ FaceJac muscl_face_jac(int lim, double wm, double w0,
   J.l1 = 1.0 + ldA - ldB;
   J.l2 = ldB;
   // right = w1 - phi(dB / (dC + E)) dC / 2
-  phi = limiter_d(lim, limiter_ratio<double>(lim, dB, dC + E), d);
+  phi = limiter_d(lim, limiter_ratio<double>(m, lim, dB, dC + E), d);
   J.right = w1 - 0.5 * phi * dC;
   double rdC = -0.5 * phi, rdB = 0.0;
   if (d != 0.0) {

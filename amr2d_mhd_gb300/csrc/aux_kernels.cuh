@@ -559,6 +559,8 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
   const TreeOp op = a.ops[opi];
   const S *D = static_cast<const S *>(a.U) + static_cast<size_t>(op.dad) * 8 * NN;
   const T E = eps_of<T>();
+  Native<T> m;
+  Native<double> m64;
   // refine.cpp:45-59 for cell c of son sq, its 8 variables
   {
     const int i = c % N, j = c / N;
@@ -573,10 +575,10 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
       const T q0 = q[jj * N + ii];
       T res = q0, r, phi;
       r = (q0 - q[jj * N + ii - 1]) / (q[jj * N + ii + 1] - q0 + E);
-      phi = T(0.25) * slope_limiter<T>(LIM_MINMOD, r, T(0)) * (q[jj * N + ii + 1] - q0);
+      phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[jj * N + ii + 1] - q0);
       res = sx == 0 ? res - phi : res + phi;
       r = (q0 - q[(jj - 1) * N + ii]) / (q[(jj + 1) * N + ii] - q0 + E);
-      phi = T(0.25) * slope_limiter<T>(LIM_MINMOD, r, T(0)) * (q[(jj + 1) * N + ii] - q0);
+      phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[(jj + 1) * N + ii] - q0);
       res = sy == 0 ? res - phi : res + phi;
       u[k] = res;
       Sn[k * NN + c] = res;
@@ -602,13 +604,13 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
   const double By_imjp = Y(-1, 1), By_jp = Y(0, 1), By_ipjp = Y(1, 1);
   double r;
   r = (Bx - Bx_jm) / (Bx_jp - Bx + EPS);
-  const double DyBxm = slope_limiter<double>(LIM_MINMOD, r, 0) * (Bx_jp - Bx);
+  const double DyBxm = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (Bx_jp - Bx);
   r = (Bx_ip - Bx_ipjm) / (Bx_ipjp - Bx_ip + EPS);
-  const double DyBxp = slope_limiter<double>(LIM_MINMOD, r, 0) * (Bx_ipjp - Bx_ip);
+  const double DyBxp = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (Bx_ipjp - Bx_ip);
   r = (By - By_im) / (By_ip - By + EPS);
-  const double DxBym = slope_limiter<double>(LIM_MINMOD, r, 0) * (By_ip - By);
+  const double DxBym = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (By_ip - By);
   r = (By_jp - By_imjp) / (By_ipjp - By_jp + EPS);
-  const double DxByp = slope_limiter<double>(LIM_MINMOD, r, 0) * (By_ipjp - By_jp);
+  const double DxByp = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (By_ipjp - By_jp);
   const double ax = (Bx_ip - Bx);
   const double by_ = -1. * ax;
   const double ay = 0.5 * (DyBxp + DyBxm);

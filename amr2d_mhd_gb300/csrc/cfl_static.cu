@@ -40,8 +40,9 @@ __global__ void __launch_bounds__(256) k_cfl_static_blocks(const double *U, cons
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = u0[k * NN + c];
     cons2prim_cell<double>(u, w, gamma);
-    const double v1 = fabs(w[0]) + fast_speed<double>(w, gamma, 5);
-    const double v2 = fabs(w[1]) + fast_speed<double>(w, gamma, 6);
+    Native<double> ar;
+    const double v1 = fabs(w[0]) + fast_speed<double>(ar, w, gamma, 5);
+    const double v2 = fabs(w[1]) + fast_speed<double>(ar, w, gamma, 6);
     // a NaN speed (e.g. a negative pressure) poisons the block's value
     m = (isnan(v1) || isnan(v2)) ? NAN : smax(smax(m, v1), v2);
   }

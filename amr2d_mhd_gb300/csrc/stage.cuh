@@ -209,6 +209,60 @@ __device__ __forceinline__ bool bulk_stage_wait(uint64_t *bar, uint32_t phase) {
   return false;
 }
 
+// MUSCL2D.cpp:24-116 for one face: W is plane 0 of the block's primitive
+// state (planes NN apart), cL the cell on its left (below it), s the cell
+// stride along its normal, yf whether that is y; bn the face's own normal
+// field (the CT override, MUSCL2D.cpp:48-51).  Returns riemann()'s code.
+template <int RECON, int FLUX, int NN, typename T, class M>
+__device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma,
+                                            T *fl) {
+  const int kn = yf ? 6 : 5;                                // normal B component
+  T wl[8], wr[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    if (k == kn) continue;
+    const T *w = W + k * NN + cL;
+    if (RECON == REC_MUSCL) {
+      const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
+      muscl_face<T>(m, lim, w0, w1, w0 - wm, w1 - w0, w2 - w1, h, wl[k], wr[k]);
+    } else if (RECON == REC_WENO3) {
+      T dummy;
+      weno3_cell<T>(m, w[-s], w[0], w[s], wl[k], dummy);
+      weno3_cell<T>(m, w[0], w[s], w[2 * s], dummy, wr[k]);
+    } else {
+      wl[k] = weno5_cell<T, false>(m, w[-2 * s], w[-s], w[0], w[s], w[2 * s]);
+      wr[k] = weno5_cell<T, true>(m, w[-s], w[0], w[s], w[2 * s], w[3 * s]);
+    }
+  }
+  wl[kn] = bn;
+  wr[kn] = bn;
+  if (!yf) return riemann<FLUX, T>(m, wl, wr, gamma, fl);
+  // riemannS.cpp:12-23, 47-55: rotate y into x and back
+  T l2[8], r2[8], f2[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) { l2[k] = wl[k]; r2[k] = wr[k]; }
+  l2[1] = wl[2]; l2[2] = wl[1]; r2[1] = wr[2]; r2[2] = wr[1];
+  l2[5] = wl[6]; l2[6] = wl[5]; r2[5] = wr[6]; r2[6] = wr[5];
+  const int rc = riemann<FLUX, T>(m, l2, r2, gamma, f2);
+#pragma unroll
+  for (int k = 0; k < 8; k++) fl[k] = f2[k];
+  fl[1] = f2[2]; fl[2] = f2[1]; fl[5] = f2[6]; fl[6] = f2[5];
+  return rc;
+}
+
+// the same with the native operators, for the rare face whose operands left
+// the range of the Soft arithmetic; a function of its own, so that its
+// registers are not the hot path's.  The flux goes to out[k * NN].
+template <int RECON, int FLUX, int NN, typename T>
+__device__ __noinline__ int face_flux_native(const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma, T *out) {
+  Native<T> m;
+  T fl[8];
+  const int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, lim, h, bn, gamma, fl);
+#pragma unroll
+  for (int k = 0; k < 8; k++) out[k * NN] = fl[k];
+  return rc;
+}
+
 // resident CTAs per SM the fused stage kernel is compiled for: the FP32
 // instantiation trades registers for occupancy (it is latency-bound)
 template <typename S> struct StageMinBlocks { static constexpr int value = 1; };
@@ -297,47 +351,19 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
     const int g = yf ? f - NF * NF : f;
     const int r = g / NF, c = g % NF;
     // cell-index stride along the face normal and the left cell of the face
-    int s, cL;
-    if (!yf) { s = 1; cL = (LO + r) * N + (LO + c); }        // face between (LO+c) and (LO+c+1), row LO+r
-    else { s = N; cL = (LO + r) * N + (LO + c); }             // face between rows LO+r and LO+r+1, column LO+c
-    const int kn = yf ? 6 : 5;                                // normal B component
-    T wl[8], wr[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      if (k == kn) continue;
-      const T *w = sW + k * NN + cL;
-      if (RECON == REC_MUSCL) {
-        const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
-        muscl_face<T>(lim, w0, w1, w0 - wm, w1 - w0, w2 - w1, static_cast<T>(yf ? task.dy : task.dx),
-                      wl[k], wr[k]);
-      } else if (RECON == REC_WENO3) {
-        T dummy;
-        weno3_cell<T>(w[-s], w[0], w[s], wl[k], dummy);
-        weno3_cell<T>(w[0], w[s], w[2 * s], dummy, wr[k]);
-      } else {
-        wl[k] = weno5_cell<T, false>(w[-2 * s], w[-s], w[0], w[s], w[2 * s]);
-        wr[k] = weno5_cell<T, true>(w[-s], w[0], w[s], w[2 * s], w[3 * s]);
-      }
-    }
-    // CT: the normal component is the face value (MUSCL2D.cpp:48-51)
+    const int s = yf ? N : 1;
+    const int cL = (LO + r) * N + (LO + c);
     const int fpos = cL + s;  // face index of the reference = the right cell
+    const T h = static_cast<T>(yf ? task.dy : task.dx);
     const T bn = static_cast<T>(yf ? By[fpos] : Bx[fpos]);
-    wl[kn] = bn;
-    wr[kn] = bn;
     T fl[8];
-    int rc;
-    if (!yf) {
-      rc = riemann<FLUX, T>(wl, wr, gamma, fl);
-    } else {  // riemannS.cpp:12-23, 47-55: rotate y into x and back
-      T l2[8], r2[8], f2[8];
+    typename ArithOf<T>::type m;
+    int rc = face_flux_of<RECON, FLUX, NN, T>(m, sW, cL, s, yf, lim, h, bn, gamma, fl);
+    if (m.failed()) {
+      T *out = (yf ? gg : ff) + fpos;
+      rc = face_flux_native<RECON, FLUX, NN, T>(sW, cL, s, yf, lim, h, bn, gamma, out);
 #pragma unroll
-      for (int k = 0; k < 8; k++) { l2[k] = wl[k]; r2[k] = wr[k]; }
-      l2[1] = wl[2]; l2[2] = wl[1]; r2[1] = wr[2]; r2[2] = wr[1];
-      l2[5] = wl[6]; l2[6] = wl[5]; r2[5] = wr[6]; r2[6] = wr[5];
-      rc = riemann<FLUX, T>(l2, r2, gamma, f2);
-#pragma unroll
-      for (int k = 0; k < 8; k++) fl[k] = f2[k];
-      fl[1] = f2[2]; fl[2] = f2[1]; fl[5] = f2[6]; fl[6] = f2[5];
+      for (int k = 0; k < 8; k++) fl[k] = out[k * NN];
     }
     if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
     bool bad = false;

@@ -1,6 +1,5 @@
-// Instantiates the stage kernel of one Riemann solver and one precision for
-// every supported (ghost layers, reconstruction) pair.  Each including .cu
-// file defines AMR_STAGE_PREC (f64 / f32), AMR_STAGE_T and AMR_STAGE_FLUX.
+// Instantiates the stage or face kernels of one Riemann solver and one precision for
+// every supported (ghost layers, reconstruction) pair.
 #pragma once
 
 #include "launch.hpp"
@@ -109,12 +108,17 @@ cudaError_t launch_faces_flux(const Method &m, const SplitArgs &a, cudaStream_t 
 
 }  // namespace amr
 
-#define AMR_STAGE_DEFINE(P, F, FLUXID, T)                                                     \
-  namespace amr {                                                                          \
+// the fused stage kernels and the face kernels of a solver and precision are
+// translation units of their own (stage_*.cu, faces_*.cu), compiled in parallel
+#define AMR_STAGE_DEFINE(P, F, FLUXID, T)                                                          \
+  namespace amr {                                                                                  \
   cudaError_t launch_stage_##P##_##F(const Method &m, const StageArgs &a, int n, cudaStream_t s) { \
-    return launch_stage_flux<FLUXID, T>(m, a, n, s);                                        \
-  }                                                                                        \
-  cudaError_t launch_faces_##P##_##F(const Method &m, const SplitArgs &a, cudaStream_t s) {  \
+    return launch_stage_flux<FLUXID, T>(m, a, n, s);                                               \
+  }                                                                                                \
+  }
+#define AMR_FACES_DEFINE(P, F, FLUXID, T)                                                   \
+  namespace amr {                                                                           \
+  cudaError_t launch_faces_##P##_##F(const Method &m, const SplitArgs &a, cudaStream_t s) { \
     return launch_faces_flux<FLUXID, T>(m, a, s);                                           \
-  }                                                                                        \
+  }                                                                                         \
   }

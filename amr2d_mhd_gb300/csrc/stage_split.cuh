@@ -103,48 +103,20 @@ __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
   const int r = g / NF, c = g % NF;
   const int s = yf ? N : 1;
   const int cL = (LO + r) * N + (LO + c);
-  const int kn = yf ? 6 : 5;
-  const T gamma = static_cast<T>(ip.gamma);
-  T wl[8], wr[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    if (k == kn) continue;
-    const S *w = W + k * NN + cL;
-    if (RECON == REC_MUSCL) {
-      const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
-      muscl_face<T>(ip.limiter, w0, w1, w0 - wm, w1 - w0, w2 - w1, static_cast<T>(yf ? task.dy : task.dx),
-                    wl[k], wr[k]);
-    } else if (RECON == REC_WENO3) {
-      T dummy;
-      weno3_cell<T>(w[-s], w[0], w[s], wl[k], dummy);
-      weno3_cell<T>(w[0], w[s], w[2 * s], dummy, wr[k]);
-    } else {
-      wl[k] = weno5_cell<T, false>(w[-2 * s], w[-s], w[0], w[s], w[2 * s]);
-      wr[k] = weno5_cell<T, true>(w[-s], w[0], w[s], w[2 * s], w[3 * s]);
-    }
-  }
+  const T gamma = static_cast<T>(ip.gamma), h = static_cast<T>(yf ? task.dy : task.dx);
   const int fpos = cL + s;
   const double *Bf = a.B + static_cast<size_t>(task.slot) * 2 * NN + (yf ? NN : 0);
   const T bn = static_cast<T>(Bf[fpos]);
-  wl[kn] = bn;
-  wr[kn] = bn;
+  S *out = static_cast<S *>(yf ? a.gg : a.ff) + base + fpos;
   T fl[8];
-  int rc;
-  if (!yf) {
-    rc = riemann<FLUX, T>(wl, wr, gamma, fl);
-  } else {
-    T l2[8], r2[8], f2[8];
+  typename ArithOf<T>::type m;
+  int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, ip.limiter, h, bn, gamma, fl);
+  if (m.failed()) {
+    rc = face_flux_native<RECON, FLUX, NN, T>(W, cL, s, yf, ip.limiter, h, bn, gamma, out);
 #pragma unroll
-    for (int k = 0; k < 8; k++) { l2[k] = wl[k]; r2[k] = wr[k]; }
-    l2[1] = wl[2]; l2[2] = wl[1]; r2[1] = wr[2]; r2[2] = wr[1];
-    l2[5] = wl[6]; l2[6] = wl[5]; r2[5] = wr[6]; r2[6] = wr[5];
-    rc = riemann<FLUX, T>(l2, r2, gamma, f2);
-#pragma unroll
-    for (int k = 0; k < 8; k++) fl[k] = f2[k];
-    fl[1] = f2[2]; fl[2] = f2[1]; fl[5] = f2[6]; fl[6] = f2[5];
+    for (int k = 0; k < 8; k++) fl[k] = out[k * NN];
   }
   if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
-  S *out = static_cast<S *>(yf ? a.gg : a.ff) + base + fpos;
   bool bad = false;
 #pragma unroll
   for (int k = 0; k < 8; k++) {

@@ -1,0 +1,90 @@
+"""The integer-pipe division and square root of the FP64 kernels
+(csrc/softfp.cuh) against IEEE division and square root, bit for bit: random
+and edge significands (all ones, powers of two, a few units around them),
+quotients and squares next to representable and halfway values, zeros, and
+exponents over the whole range, where the routines must either report that
+the operands are outside theirs or be right.  On the CPU with seeds displaced
+by MUFU's error bounds, on the GPU with MUFU itself."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "amr2d_mhd_gb300", "csrc")
+
+
+def check_lib(gpu):
+    src = os.path.join(HERE, "softfp_check.cu")
+    out = os.path.join(HERE, "_build", "softfp_%s.so" % ("gpu" if gpu else "cpu"))
+    if not os.path.exists(out) or os.path.getmtime(out) < max(os.path.getmtime(src),
+                                                             os.path.getmtime(os.path.join(CSRC, "softfp.cuh"))):
+        os.makedirs(os.path.dirname(out), exist_ok=True)
+        cmd = ([shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc", "-shared", "-Xcompiler", "-fPIC", "-gencode",
+                "arch=compute_103a,code=sm_103a", "-fmad=false"] if gpu else
+               ["g++", "-x", "c++", "-shared", "-fPIC", "-ffp-contract=off"])
+        subprocess.check_call(cmd + ["-O2", "-std=c++17", "-I" + CSRC, src, "-o", out])
+    L = ctypes.CDLL(out)
+    L.softfp_check.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_long, ctypes.c_double, ctypes.c_void_p,
+                               ctypes.c_void_p]
+    return L
+
+
+def operands(n, seed):
+    """n (a, b): significands and exponents of every kind the docstring names."""
+    g = np.random.default_rng(seed)
+
+    def mant():
+        m = g.integers(0, 1 << 52, n, dtype=np.uint64)
+        k = g.integers(0, 8, n)
+        few, bit = m & 7, np.uint64(1) << (m % 52)
+        ones = np.uint64((1 << 52) - 1)
+        return np.select([k == 0, k == 1, k == 2, k == 3, k == 4, k == 5], [few, ones - few, bit, ones ^ bit,
+                                                                            m & ~(bit - np.uint64(1)),
+                                                                            m | (bit - np.uint64(1))], m)
+
+    def num():
+        e = np.where(g.random(n) < 0.8, g.integers(963, 1083, n), g.integers(0, 2048, n)).astype(np.uint64)
+        s = g.integers(0, 2, n, dtype=np.uint64) << np.uint64(63)
+        return (s | e << np.uint64(52) | mant()).view(np.float64)
+    a, b = num(), num()
+    with np.errstate(all="ignore"):
+        pick = g.integers(0, 4, n)
+        near = np.where(pick == 1, a * b, np.where(pick == 2, b * b, a))  # quotient near a, root near |b|
+        near = (near.view(np.int64) + np.where(pick > 0, g.integers(-1, 2, n), 0)).view(np.float64)
+    near[g.random(n) < 0.02] = 0.0
+    near[g.random(n) < 0.02] = -0.0
+    return near, b
+
+
+def compare(L, n, seed, rel=0.0):
+    a, b = operands(n, seed)
+    out, bad = np.zeros((4, n)), np.zeros(n, np.uint8)
+    assert L.softfp_check(a.ctypes.data, b.ctypes.data, n, rel, out.ctypes.data, bad.ctypes.data) == 0
+    with np.errstate(all="ignore"):
+        want = [a / b, np.sqrt(a), a / 3.0, a / 6.0]
+    for k, w in enumerate(want):
+        ok = (bad >> k & 1) == 0
+        assert np.array_equal(out[k][ok].view(np.int64), w[ok].view(np.int64)), k
+        # operands of ordinary size, and zeros, are never refused (sqrt: of either zero or positive numbers)
+        with np.errstate(all="ignore"):
+            mid = (np.abs(a) > 1e-150) & (np.abs(a) < 1e150) & (np.abs(b) > 1e-150) & (np.abs(b) < 1e150)
+        mid |= (a == 0) & (np.abs(b) > 1e-300) & (np.abs(b) < 1e300)
+        if k == 1:
+            mid &= a >= 0
+        assert ok[mid].all(), k
+
+
+@pytest.mark.parametrize("rel", [0.0, 2.0 ** -22.9, -2.0 ** -22.9])
+def test_soft_division_and_root_on_the_cpu(rel):
+    compare(check_lib(False), 1 << 20, 7, rel)
+
+
+@pytest.mark.gpu
+def test_soft_division_and_root_on_the_gpu(gpu):
+    L = check_lib(True)
+    for seed in range(8):
+        compare(L, 1 << 20, seed)

@@ -227,18 +227,18 @@ __device__ __forceinline__ double limiter_d(int lim, double r, double &d) {
 // first order, right = r0 W[m] + r1 W[m+1] + r2 W[m+2]
 struct FaceJac { double left, right, l0, l1, l2, r0, r1, r2; };
 
-__device__ __forceinline__ FaceJac muscl_face_jac(int lim, double wm, double w0, double w1, double w2) {
+template <class M>
+__device__ __forceinline__ FaceJac muscl_face_jac(M &m, int lim, double wm, double w0, double w1, double w2) {
   const double E = 1.0E-15;
   const double dA = w0 - wm, dB = w1 - w0, dC = w2 - w1;
   FaceJac J;
-  Native<double> m;
   double d;
   // left = w0 + phi(dB / (dA + E)) dA / 2
   double phi = limiter_d(lim, limiter_ratio<double>(m, lim, dB, dA + E), d);
   J.left = w0 + 0.5 * phi * dA;
   double ldA = 0.5 * phi, ldB = 0.0;
   if (d != 0.0) {
-    const double inv = 1.0 / (dA + E), q = 0.5 * dA * d * inv;
+    const double inv = m.div(1.0, dA + E), q = 0.5 * dA * d * inv;
     ldA -= q * dB * inv;
     ldB = q;
   }
@@ -250,7 +250,7 @@ __device__ __forceinline__ FaceJac muscl_face_jac(int lim, double wm, double w0,
   J.right = w1 - 0.5 * phi * dC;
   double rdC = -0.5 * phi, rdB = 0.0;
   if (d != 0.0) {
-    const double inv = 1.0 / (dC + E), q = 0.5 * dC * d * inv;
+    const double inv = m.div(1.0, dC + E), q = 0.5 * dC * d * inv;
     rdC += q * dB * inv;
     rdB = -q;
   }
@@ -268,10 +268,11 @@ struct SideAD {
   double irho, e, pt, A, C, T, D, cf;
 };
 
-__device__ __forceinline__ void side_fwd(const double *w, double g, double ig1, SideAD &S) {
+template <class M>
+__device__ __forceinline__ void side_fwd(M &m, const double *w, double g, double ig1, SideAD &S) {
   const double rho = w[0], u = w[1], v = w[2], z = w[3], p = w[4], bx = w[5], by = w[6], bz = w[7];
   const double b2 = bx * bx + by * by + bz * bz, t2 = by * by + bz * bz;
-  S.irho = 1.0 / rho;
+  S.irho = m.div(1.0, rho);
   S.e = p * ig1 + 0.5 * rho * (u * u + v * v + z * z) + 0.5 * b2;
   S.pt = p + 0.5 * b2;
   S.q[0] = rho; S.q[1] = rho * u; S.q[2] = rho * v; S.q[3] = rho * z;
@@ -279,12 +280,13 @@ __device__ __forceinline__ void side_fwd(const double *w, double g, double ig1, 
   S.A = g * p * S.irho;
   S.C = b2 * S.irho;
   S.T = t2 * S.irho;
-  S.D = sqrt((S.C - S.A) * (S.C - S.A) + 4.0 * S.A * S.T);
-  S.cf = sqrt(0.5 * (S.C + S.A + S.D));
+  S.D = m.root((S.C - S.A) * (S.C - S.A) + 4.0 * S.A * S.T);
+  S.cf = m.root(0.5 * (S.C + S.A + S.D));
 }
 
 // adds d/dw of lF.F + lq.q + lcf.cf of one side to lw
-__device__ __forceinline__ void side_adj(const double *w, double g, double ig1, const SideAD &S, const double *lF,
+template <class M>
+__device__ __forceinline__ void side_adj(M &m, const double *w, double g, double ig1, const SideAD &S, const double *lF,
                                          const double *lq, double lcf, double *lw) {
   const double rho = w[0], u = w[1], v = w[2], z = w[3], bx = w[5], by = w[6], bz = w[7];
   const double le = lq[4] + lF[4] * u;     // adjoint of e
@@ -303,10 +305,10 @@ __device__ __forceinline__ void side_adj(const double *w, double g, double ig1, 
   double lby = lq[6] + lb * by - bx * lF[2] - bx * v * lF[4] + u * lF[6];
   double lbz = lq[7] + lb * bz - bx * lF[3] - bx * z * lF[4] + u * lF[7];
   if (lcf != 0.0) {  // cf^2 = (C + A + D) / 2, D^2 = (C - A)^2 + 4 A T
-    const double k = lcf / (4.0 * S.cf);
+    const double k = m.div(lcf, 4.0 * S.cf);
     double lA = k, lC = k, lT = 0.0;
     if (S.D > 0.0) {
-      const double kD = k / S.D;
+      const double kD = m.div(k, S.D);
       lA += kD * (2.0 * S.T - (S.C - S.A));
       lC += kD * (S.C - S.A);
       lT = kD * 2.0 * S.A;
@@ -324,12 +326,13 @@ __device__ __forceinline__ void side_adj(const double *w, double g, double ig1, 
 
 // riemannS.cpp:58-116 (Rusanov) transposed for one face in the x frame:
 // f = (FL + FR)/2 - max(cfL + |uL|, cfR + |uR|) (qR - qL)/2
-__device__ __forceinline__ void rusa_adj(const double *wL, const double *wR, double g, const double *lf,
+template <class M>
+__device__ __forceinline__ void rusa_adj(M &m, const double *wL, const double *wR, double g, const double *lf,
                                          double *lwL, double *lwR) {
-  const double ig1 = 1.0 / (g - 1.0);
+  const double ig1 = m.div(1.0, g - 1.0);
   SideAD L, R;
-  side_fwd(wL, g, ig1, L);
-  side_fwd(wR, g, ig1, R);
+  side_fwd(m, wL, g, ig1, L);
+  side_fwd(m, wR, g, ig1, R);
   const double a = L.cf + fabs(wL[1]), b = R.cf + fabs(wR[1]);
   const double im = smax(a, b);
   double lF[8], lqL[8], lqR[8], lim = 0.0;
@@ -345,8 +348,8 @@ __device__ __forceinline__ void rusa_adj(const double *wL, const double *wR, dou
   for (int k = 0; k < 8; k++) { lwL[k] = 0.0; lwR[k] = 0.0; }
   lwL[1] += la * sgn(wL[1]);
   lwR[1] += lb * sgn(wR[1]);
-  side_adj(wL, g, ig1, L, lF, lqL, la, lwL);
-  side_adj(wR, g, ig1, R, lF, lqR, lb, lwR);
+  side_adj(m, wL, g, ig1, L, lF, lqL, la, lwL);
+  side_adj(m, wR, g, ig1, R, lF, lqR, lb, lwR);
 }
 
 // MUSCL2D.cpp:24-116 + riemannS + the residual (main.cpp:147-157)
@@ -354,12 +357,13 @@ __device__ __forceinline__ void rusa_adj(const double *wL, const double *wR, dou
 // the residual of the face's two cells) becomes the adjoint of the two
 // reconstructed states, of the normal face field (added to aB) and, through
 // the MUSCL Jacobian, of the primitive state of the four stencil cells (C).
-template <int NG>
-__global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
+// Bound by the FP64 pipe; with Soft divisions and roots (softfp.cuh) 303 us
+// for 256 blocks, 387 before.
+template <int NG, class M>
+__device__ __forceinline__ bool face_adj(const StageAdjArgs &a, size_t e) {
+  M ar;
   using G = Geo<NG>;
   constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI, NF = G::NF, PER = 2 * NF * NF;
-  const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= static_cast<size_t>(a.ntasks) * PER) return;
   const int t = static_cast<int>(e / PER), f = static_cast<int>(e % PER);
   const LeafTask task = a.tasks[t];
   const InstParams ip = a.inst[task.inst];
@@ -380,15 +384,15 @@ __global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
   for (int k = 0; k < 8; k++) {
     if (k == kn) { wl[k] = wr[k] = bn; continue; }
     const double *w = W + k * NN + cL;
-    J[k] = muscl_face_jac(lim, w[-s], w[0], w[s], w[2 * s]);
+    J[k] = muscl_face_jac(ar, lim, w[-s], w[0], w[s], w[2 * s]);
     wl[k] = J[k].left;
     wr[k] = J[k].right;
   }
   // flux adjoint: CT2D part after the fill, plus the residual of cells m
   // (+1/h) and m+1 (-1/h) when they lie in [LO, HI]
   const double sdt = (a.step == 1 ? 1.0 : 0.5) * ip.dt;
-  const double h = yf ? (task.inv_dy != 0.0 ? task.inv_dy : 1.0 / task.dy)
-                      : (task.inv_dx != 0.0 ? task.inv_dx : 1.0 / task.dx);
+  const double h = yf ? (task.inv_dy != 0.0 ? task.inv_dy : ar.div(1.0, task.dy))
+                      : (task.inv_dx != 0.0 ? task.inv_dx : ar.div(1.0, task.dx));
   const int m = LO + (yf ? r : c);          // cell index along the face normal
   const bool hi_in = m + 1 <= HI;
   const double *af = (yf ? a.aG : a.aF) + base + fpos;
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
   }
   double lwl[8], lwr[8];
   if (!yf) {
-    rusa_adj(wl, wr, ip.gamma, lf, lwl, lwr);
+    rusa_adj(ar, wl, wr, ip.gamma, lf, lwl, lwr);
   } else {  // riemannS.cpp:12-23 / 47-55: swap (u, v) and (Bx, By)
     double l2[8], r2[8], f2[8], a2[8], b2[8];
 #pragma unroll
@@ -410,12 +414,13 @@ __global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
     l2[1] = wl[2]; l2[2] = wl[1]; r2[1] = wr[2]; r2[2] = wr[1];
     l2[5] = wl[6]; l2[6] = wl[5]; r2[5] = wr[6]; r2[6] = wr[5];
     f2[1] = lf[2]; f2[2] = lf[1]; f2[5] = lf[6]; f2[6] = lf[5];
-    rusa_adj(l2, r2, ip.gamma, f2, a2, b2);
+    rusa_adj(ar, l2, r2, ip.gamma, f2, a2, b2);
 #pragma unroll
     for (int k = 0; k < 8; k++) { lwl[k] = a2[k]; lwr[k] = b2[k]; }
     lwl[1] = a2[2]; lwl[2] = a2[1]; lwr[1] = b2[2]; lwr[2] = b2[1];
     lwl[5] = a2[6]; lwl[6] = a2[5]; lwr[5] = b2[6]; lwr[6] = b2[5];
   }
+  if (ar.failed()) return false;  // nothing stored yet
   // the normal component of both states is the face field (MUSCL2D.cpp:48-51)
   a.aB[static_cast<size_t>(task.slot) * 2 * NN + (yf ? NN : 0) + fpos] += lwl[kn] + lwr[kn];
   const int d = yf ? 1 : 0;
@@ -430,6 +435,20 @@ __global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
     c2[k * NN] = J[k].l2 * L + J[k].r1 * R;    // cell m+1
     c3[k * NN] = J[k].r2 * R;                  // cell m+2
   }
+  return true;
+}
+
+template <int NG>
+__device__ __noinline__ void face_adj_native(const StageAdjArgs &a, size_t e) {
+  face_adj<NG, Native<double>>(a, e);
+}
+
+template <int NG>
+__global__ void __launch_bounds__(128) k_faces_adj(StageAdjArgs a) {
+  constexpr int PER = 2 * Geo<NG>::NF * Geo<NG>::NF;
+  const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= static_cast<size_t>(a.ntasks) * PER) return;
+  if (!face_adj<NG, Soft>(a, e)) face_adj_native<NG>(a, e);
 }
 
 // Per cell: the primitive-state adjoint gathered from the (up to 8) faces
@@ -471,10 +490,12 @@ __global__ void __launch_bounds__(256) k_cells_adj(StageAdjArgs a) {
   const double rho = W[c], u = W[NN + c], v = W[2 * NN + c], z = W[3 * NN + c];
   const double gm = gamma - 1.0;
   double g[8];
-  g[0] = lw[0] - (lw[1] * u + lw[2] * v + lw[3] * z) / rho + lw[4] * gm * 0.5 * (u * u + v * v + z * z);
-  g[1] = lw[1] / rho - lw[4] * gm * u;
-  g[2] = lw[2] / rho - lw[4] * gm * v;
-  g[3] = lw[3] / rho - lw[4] * gm * z;
+  evaluate<double>([&](auto &m) {
+    g[0] = lw[0] - m.div(lw[1] * u + lw[2] * v + lw[3] * z, rho) + lw[4] * gm * 0.5 * (u * u + v * v + z * z);
+    g[1] = m.div(lw[1], rho) - lw[4] * gm * u;
+    g[2] = m.div(lw[2], rho) - lw[4] * gm * v;
+    g[3] = m.div(lw[3], rho) - lw[4] * gm * z;
+  });
   g[4] = lw[4] * gm;
 #pragma unroll
   for (int k = 5; k < 8; k++) g[k] = lw[k] - lw[4] * gm * W[k * NN + c];

@@ -312,6 +312,9 @@ __global__ void __launch_bounds__(128) k_diffuse(CtArgs a) {
 // NaN trap on every cell, as k_prim), then one thread per interior cell
 // forms the wave speeds and the criterion from them (FP64 for the FP64 path;
 // the FP32 path computes the cell values in FP32 and reduces them in FP64).
+// The FP64 form was bound by the FP64 pipe; with divisions, roots and the
+// criterion's maxima on the integer pipe (softfp.cuh) it takes 25 us for the
+// 196 leaves of a rotor, 60 before.
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -377,36 +380,28 @@ __global__ void __launch_bounds__(256) k_dt_cell(DtArgs a) {
   T w[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) w[k] = W[k * NN + c];
-  // wavespeeds (misc.cpp:71-79) for norm 5 and 6; ca and a are the same
-  // values in both calls.  lambda1 takes |rho| (main.cpp:222), lambda2 |u|.
-  const T ca = sqrt((w[5] * w[5] + w[6] * w[6] + w[7] * w[7]) / w[0]);
-  const T as = sqrt(g * w[4] / w[0]);
-  T cf[2];
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const T can = sqrt((w[5 + q] * w[5 + q]) / w[0]);
-    const T i0 = (ca * ca) + (as * as), i1 = (ca * ca) - (as * as);
-    cf[q] = sqrt(T(0.5) * (i0 + sqrt(i1 * i1 + T(4.) * (as * as) * ((ca * ca) - (can * can)))));
-  }
-  // the maxima in the storage type, widened to FP64 once per warp: the
-  // widening is exact and monotonic, so this equals the maximum of the
-  // widened values (and keeps FP32 maxima off the FP64 pipe)
-  T lamT = smax(fabs(w[0]) + cf[0], fabs(w[1]) + cf[1]);
-  T grT = T(0.);
-  if (a.want_grad) {
+  // wavespeeds (misc.cpp:71-79) for norm 5 and 6; lambda1 takes |rho|
+  // (main.cpp:222), lambda2 |u|.  The maxima in the storage type, widened to
+  // FP64 once per warp: the widening is exact and monotonic, so this equals
+  // the maximum of the widened values (and keeps FP32 maxima off the FP64 pipe).
+  T lamT = T(0.), grT = T(0.);
+  evaluate<T>([&](auto &m) {
+    T cf[2];
+    fast_speeds<T>(m, w, g, cf);
+    lamT = smax(fabs(w[0]) + cf[0], fabs(w[1]) + cf[1]);
+    grT = T(0.);
+    if (!a.want_grad) return;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int v = q == 0 ? 4 : (q == 1 ? 0 : q + 3);   // p, rho, Bx, By
       const S *x = W + v * NN + c;
       const T c0 = x[0];
-      const T dm = mmax(static_cast<T>(EPS), fabs(c0));
-      T d1 = fabs(x[1] - c0);
-      T d2 = mmax(d1, fabs(x[-1] - c0));
-      d1 = mmax(d2, fabs(x[N] - c0));
-      d2 = mmax(d1, fabs(x[-N] - c0));
-      grT = mmax(grT, d2 / dm);
+      const T dm = m.most(static_cast<T>(EPS), fabs(c0));
+      const T d1 = m.most(fabs(x[1] - c0), fabs(x[-1] - c0));
+      const T d2 = m.most(fabs(x[N] - c0), fabs(x[-N] - c0));
+      grT = m.most(grT, m.div(m.most(d1, d2), dm));
     }
-  }
+  });
   const double lam = static_cast<double>(warp_max_t(lamT));
   const double gr = static_cast<double>(warp_max_t(grT));
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -542,7 +537,8 @@ struct TreeOpArgs {
 // U2W("refine") on the sons, then refineBi_CT.cpp:4-74 for the face field.
 // Work is spread over many CTAs: CTA (op, son, chunk) takes kRefineChunk
 // cells of one son, one thread per cell (8 variables and 2 face components),
-// so the FP64 divisions of a refined block run on many SMs at once.
+// so the work of a refined block runs on many SMs at once; the limiter ratios
+// are Soft divisions (softfp.cuh) on the FP64 path.
 constexpr int kRefineChunk = 128;
 template <int NG> __host__ __device__ constexpr int refine_chunks() {
   return (Geo<NG>::NN + kRefineChunk - 1) / kRefineChunk;
@@ -559,8 +555,6 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
   const TreeOp op = a.ops[opi];
   const S *D = static_cast<const S *>(a.U) + static_cast<size_t>(op.dad) * 8 * NN;
   const T E = eps_of<T>();
-  Native<T> m;
-  Native<double> m64;
   // refine.cpp:45-59 for cell c of son sq, its 8 variables
   {
     const int i = c % N, j = c / N;
@@ -569,20 +563,23 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
     const int jj = (sq & 2) ? (j - NG + 2) / 2 + n2 : (j + NG) / 2;
     S *Sn = static_cast<S *>(a.U) + static_cast<size_t>(op.son[sq]) * 8 * NN;
     T u[8];
+    evaluate<T>([&](auto &m) {
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const S *q = D + k * NN;
-      const T q0 = q[jj * N + ii];
-      T res = q0, r, phi;
-      r = (q0 - q[jj * N + ii - 1]) / (q[jj * N + ii + 1] - q0 + E);
-      phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[jj * N + ii + 1] - q0);
-      res = sx == 0 ? res - phi : res + phi;
-      r = (q0 - q[(jj - 1) * N + ii]) / (q[(jj + 1) * N + ii] - q0 + E);
-      phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[(jj + 1) * N + ii] - q0);
-      res = sy == 0 ? res - phi : res + phi;
-      u[k] = res;
-      Sn[k * NN + c] = res;
-    }
+      for (int k = 0; k < 8; k++) {
+        const S *q = D + k * NN;
+        const T q0 = q[jj * N + ii];
+        T res = q0, r, phi;
+        r = m.div(q0 - q[jj * N + ii - 1], q[jj * N + ii + 1] - q0 + E);
+        phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[jj * N + ii + 1] - q0);
+        res = sx == 0 ? res - phi : res + phi;
+        r = m.div(q0 - q[(jj - 1) * N + ii], q[(jj + 1) * N + ii] - q0 + E);
+        phi = T(0.25) * slope_limiter<T>(m, LIM_MINMOD, r, T(0)) * (q[(jj + 1) * N + ii] - q0);
+        res = sy == 0 ? res - phi : res + phi;
+        u[k] = res;
+      }
+    });
+#pragma unroll
+    for (int k = 0; k < 8; k++) Sn[k * NN + c] = u[k];
     // U2W("refine") pressure trap (refine.cpp:70-82)
     T w[8];
     cons2prim_cell<S>(u, w, a.inst[op.inst].gamma);
@@ -602,15 +599,16 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
   const double Bx_ip = X(1, 0), Bx_ipjm = X(1, -1), Bx_ipjp = X(1, 1);
   const double By_im = Y(-1, 0), By = Y(0, 0), By_ip = Y(1, 0);
   const double By_imjp = Y(-1, 1), By_jp = Y(0, 1), By_ipjp = Y(1, 1);
-  double r;
-  r = (Bx - Bx_jm) / (Bx_jp - Bx + EPS);
-  const double DyBxm = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (Bx_jp - Bx);
-  r = (Bx_ip - Bx_ipjm) / (Bx_ipjp - Bx_ip + EPS);
-  const double DyBxp = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (Bx_ipjp - Bx_ip);
-  r = (By - By_im) / (By_ip - By + EPS);
-  const double DxBym = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (By_ip - By);
-  r = (By_jp - By_imjp) / (By_ipjp - By_jp + EPS);
-  const double DxByp = slope_limiter<double>(m64, LIM_MINMOD, r, 0) * (By_ipjp - By_jp);
+  double DyBxm = 0, DyBxp = 0, DxBym = 0, DxByp = 0;
+  evaluate<double>([&](auto &m) {
+    auto slope = [&](double lo, double mid, double hi) {
+      return slope_limiter<double>(m, LIM_MINMOD, m.div(mid - lo, hi - mid + EPS), 0) * (hi - mid);
+    };
+    DyBxm = slope(Bx_jm, Bx, Bx_jp);
+    DyBxp = slope(Bx_ipjm, Bx_ip, Bx_ipjp);
+    DxBym = slope(By_im, By, By_ip);
+    DxByp = slope(By_imjp, By_jp, By_ipjp);
+  });
   const double ax = (Bx_ip - Bx);
   const double by_ = -1. * ax;
   const double ay = 0.5 * (DyBxp + DyBxm);

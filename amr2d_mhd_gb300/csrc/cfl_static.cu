@@ -23,6 +23,10 @@ constexpr int kCflStaticMaxBlocks = 1 << 16;
 // per-block min(dx,dy)/lambda_b of the last call; shared by every call
 static __device__ __align__(256) double g_cfl_scratch[kCflStaticMaxBlocks];
 
+// Bound by the FP64 pipe (83 % busy): about 80 FP64 instructions per cell
+// with the divisions and square roots on the integer pipe (softfp.cuh), 240
+// with the compiler's; 20011 blocks take 0.77 ms, 2.25 ms before, where the
+// bytes would take 0.05 ms.
 // main.cpp:211-228 for one block of the dense array: lambda1 takes |rho| +
 // c_f,x (W[..][0], main.cpp:222) and lambda2 |u| + c_f,y (:224) over the
 // interior cells
@@ -40,9 +44,13 @@ __global__ void __launch_bounds__(256) k_cfl_static_blocks(const double *U, cons
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = u0[k * NN + c];
     cons2prim_cell<double>(u, w, gamma);
-    Native<double> ar;
-    const double v1 = fabs(w[0]) + fast_speed<double>(ar, w, gamma, 5);
-    const double v2 = fabs(w[1]) + fast_speed<double>(ar, w, gamma, 6);
+    double v1 = 0, v2 = 0;
+    evaluate<double>([&](auto &ar) {
+      double cf[2];
+      fast_speeds<double>(ar, w, gamma, cf);
+      v1 = fabs(w[0]) + cf[0];
+      v2 = fabs(w[1]) + cf[1];
+    });
     // a NaN speed (e.g. a negative pressure) poisons the block's value
     m = (isnan(v1) || isnan(v2)) ? NAN : smax(smax(m, v1), v2);
   }

@@ -199,6 +199,19 @@ __device__ __forceinline__ T fast_speed(M &m, const T *w, T gamma, int norm) {
   return m.root(T(0.5) * (i0 + m.root(i1 * i1 + T(4.) * (a * a) * ((ca * ca) - (can * can)))));
 }
 
+// the same for norm 5 (x) and 6 (y), whose first two terms are the same values
+template <typename T, class M>
+__device__ __forceinline__ void fast_speeds(M &m, const T *w, T gamma, T *cf) {
+  const T ca = m.root(m.div(w[5] * w[5] + w[6] * w[6] + w[7] * w[7], w[0]));
+  const T a = m.root(m.div(gamma * w[4], w[0]));
+  const T i0 = (ca * ca) + (a * a), i1 = (ca * ca) - (a * a);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const T can = m.root(m.div(w[5 + q] * w[5 + q], w[0]));
+    cf[q] = m.root(T(0.5) * (i0 + m.root(i1 * i1 + T(4.) * (a * a) * ((ca * ca) - (can * can)))));
+  }
+}
+
 // conserved state, physical flux, enthalpy, total pressure and energy of one
 // side (riemannS.cpp:59-108)
 template <typename T>

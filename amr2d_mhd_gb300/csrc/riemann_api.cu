@@ -21,8 +21,8 @@ __global__ void k_riemann_pairs(const double *wL, const double *wR, double gamma
     l[1] = wL[8 * q + 2]; l[2] = wL[8 * q + 1]; r[1] = wR[8 * q + 2]; r[2] = wR[8 * q + 1];
     if (mag_field) { l[5] = wL[8 * q + 6]; l[6] = wL[8 * q + 5]; r[5] = wR[8 * q + 6]; r[6] = wR[8 * q + 5]; }
   }
-  Native<double> m;
-  const int rc = riemann<FLUX, double>(m, l, r, gamma, f);
+  int rc = 0;
+  evaluate<double>([&](auto &m) { rc = riemann<FLUX, double>(m, l, r, gamma, f); });
   double o[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) o[k] = f[k];

@@ -242,6 +242,9 @@ struct Native {
   __device__ __forceinline__ T div(T a, T b) { return a / b; }
   __device__ __forceinline__ T root(T x) { return sqrt(x); }
   template <int B> __device__ __forceinline__ T by(T a) { return a / T(B); }
+  // the larger of two values that are not negative; Soft compares the bits,
+  // where a NaN counts as the largest (and the division it reaches fails)
+  __device__ __forceinline__ T most(T a, T b) { return a > b ? a : b; }
   __device__ __forceinline__ bool failed() const { return false; }
 };
 struct Soft {
@@ -249,10 +252,23 @@ struct Soft {
   __device__ __forceinline__ double div(double a, double b) { return div_rn(a, b, bad); }
   __device__ __forceinline__ double root(double x) { return sqrt_rn(x, bad); }
   template <int B> __device__ __forceinline__ double by(double a) { return div_by<B>(a, bad); }
+  __device__ __forceinline__ double most(double a, double b) { return f64_bits(a) > f64_bits(b) ? a : b; }
   __device__ __forceinline__ bool failed() const { return bad; }
 };
 template <typename T> struct ArithOf { using type = Native<T>; };
 template <> struct ArithOf<double> { using type = Soft; };
+
+// f(m) with the arithmetic of T, repeated with Native where that failed; f
+// only writes values that the repetition overwrites
+template <typename T, class F>
+__device__ __forceinline__ void evaluate(F &&f) {
+  typename ArithOf<T>::type m;
+  f(m);
+  if (m.failed()) {
+    Native<T> n;
+    f(n);
+  }
+}
 #endif
 
 }  // namespace amr

@@ -65,17 +65,21 @@ constexpr double kPressureFloor = 1.0e-10;
 template <typename S>
 __device__ __forceinline__ void cons2prim_cell(const S *u, S *w, double gamma);
 
-template <>
-__device__ __forceinline__ void cons2prim_cell<double>(const double *u, double *w, double g) {
+template <class M>
+__device__ __forceinline__ void cons2prim_f64(M &m, const double *u, double *w, double g) {
   w[0] = u[0];
-  w[1] = u[1] / u[0];
-  w[2] = u[2] / u[0];
-  w[3] = u[3] / u[0];
+  w[1] = m.div(u[1], u[0]);
+  w[2] = m.div(u[2], u[0]);
+  w[3] = m.div(u[3], u[0]);
   double p = (g - 1) * (u[4] - 0.5 * w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]));
   w[5] = u[5];
   w[6] = u[6];
   w[7] = u[7];
   w[4] = p - (g - 1) * (0.5 * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]));
+}
+template <>
+__device__ __forceinline__ void cons2prim_cell<double>(const double *u, double *w, double g) {
+  evaluate<double>([&](auto &m) { cons2prim_f64(m, u, w, g); });
 }
 
 // a^2 + b^2 + c^2 of FP32 values as an unevaluated sum hi + lo, exact to
@@ -391,8 +395,10 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
     T res = T(0.);
     if (i >= LO && i <= HI && j >= LO && j <= HI) {
       const int cx = i - LO, r = j - LO;
-      res = (sFx[(k * NF + r) * NFX + cx + 1] - sFx[(k * NF + r) * NFX + cx]) / dx +
-            (sFy[(k * NFX + r + 1) * NF + cx] - sFy[(k * NFX + r) * NF + cx]) / dy;
+      evaluate<T>([&](auto &m) {
+        res = m.div(sFx[(k * NF + r) * NFX + cx + 1] - sFx[(k * NF + r) * NFX + cx], dx) +
+              m.div(sFy[(k * NFX + r + 1) * NF + cx] - sFy[(k * NFX + r) * NF + cx], dy);
+      });
     }
     const T q = KEEPU ? sU[e] : Q[e];
     if (a.step == 1) out[e] = q - dt * res;                         // Us = U - dt res

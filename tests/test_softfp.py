@@ -88,3 +88,29 @@ def test_soft_division_and_root_on_the_gpu(gpu):
     L = check_lib(True)
     for seed in range(8):
         compare(L, 1 << 20, seed)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flux", ["RUSA", "HLLE", "HLLC", "HLLD"])
+def test_riemann_with_operands_outside_the_soft_range(gpu, flux):
+    """Face states with zero, subnormal, tiny and huge components, where the
+    kernel falls back to the native operators, against the oracle bit for bit."""
+    from oracle import pyoracle as P
+    g = np.random.default_rng(11)
+    n = 4000
+    w = g.normal(0.0, 1.0, (2, n, 8))
+    w[..., 0], w[..., 4] = g.uniform(0.1, 3.0, (2, n)), g.uniform(0.05, 2.0, (2, n))
+    scale = g.choice([0.0, 1e-320, 1e-310, 1e-160, 1e-20, 1.0, 1.0, 1.0, 1e90], (2, n, 8))
+    cols = [1, 2, 3, 5, 6, 7]
+    w[..., cols] *= scale[..., cols]
+    w[..., 4] *= g.choice([1e-300, 1e-20, 1.0, 1.0], (2, n))
+    w[1, :, 5] = w[0, :, 5]
+    out, st = gpu.riemann(flux, w[0], w[1], 5.0 / 3.0)
+    names = ["RUSA", "HLLE", "HLLC", "HLLD"]
+    want = np.zeros(8)
+    for i in range(n):
+        l, r = np.ascontiguousarray(w[0, i]), np.ascontiguousarray(w[1, i])
+        rc = P.lib().oracle_riemann(names.index(flux), l.ctypes.data, r.ctypes.data, 5.0 / 3.0, 0, want.ctypes.data)
+        assert (st[i] != 0) == (rc != 0), i
+        if rc == 0:
+            assert np.array_equal(out[i], want, equal_nan=True), (i, out[i], want)

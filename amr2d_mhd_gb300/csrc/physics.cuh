@@ -42,6 +42,31 @@ __device__ __forceinline__ bool bits_nan(double x) {
 }
 __device__ __forceinline__ bool bits_nan(float x) { return (__float_as_uint(x) & 0x7fffffffu) > 0x7f800000u; }
 
+// sgn() of a double from its bits
+template <> __device__ __forceinline__ double sgn<double>(double v) {
+  return bits_zero(v) || bits_nan(v) ? 0.0 : (__double2hiint(v) < 0 ? -1.0 : 1.0);
+}
+
+// slopelimiter.cpp:14-18 and :23-27, max(0, min(1, r)) and max(0, min(2r,
+// (1+r)/2, 2)) with the macros of defs.hpp.  The Soft forms give the same
+// bits: a negative r gives +0 and -0 gives -0; the rest are comparisons of
+// values that are not negative.
+template <typename T>
+__device__ __forceinline__ T minmod_of(Native<T> &, T r) { return mmax(T(0), mmin(T(1), r)); }
+__device__ __forceinline__ double minmod_of(Soft &m, double r) {
+  const double c = m.least(r, 1.0);
+  return __double2hiint(r) < 0 ? (m.nonzero(r) ? 0.0 : r) : c;
+}
+template <typename T>
+__device__ __forceinline__ T mc_of(Native<T> &, T r) {
+  const T a = T(2) * r, b = T(0.5) * (T(1) + r);
+  return mmax(T(0), mmin(mmin(a, b), T(2)));
+}
+__device__ __forceinline__ double mc_of(Soft &m, double r) {
+  const double c = m.least(m.least(m.twice(r), m.half(1.0 + fabs(r))), 2.0);
+  return __double2hiint(r) < 0 ? (m.nonzero(r) ? 0.0 : r) : c;
+}
+
 // slopelimiter.cpp:6-54
 template <typename T, class M>
 __device__ __forceinline__ T slope_limiter(M &m, int lim, T r, T eta) {
@@ -49,7 +74,7 @@ __device__ __forceinline__ T slope_limiter(M &m, int lim, T r, T eta) {
   switch (lim) {
     case LIM_1ST: return T(0);
     case LIM_NOSL: return r;
-    case LIM_MINMOD: { T a = mmin(T(1), r); return mmax(T(0), a); }
+    case LIM_MINMOD: return minmod_of(m, r);
     case LIM_VANLEER: return m.div(fabs(r) + r, T(1) + fabs(r));
     case LIM_SUPERBEE: {
       T a = T(2) * r;
@@ -58,12 +83,7 @@ __device__ __forceinline__ T slope_limiter(M &m, int lim, T r, T eta) {
       T c = mmax(a, b);
       return mmax(T(0), c);
     }
-    case LIM_MC: {
-      T a = T(2) * r, b = T(0.5) * (T(1) + r);
-      T c = mmin(a, b);
-      a = mmin(c, T(2));
-      return mmax(T(0), a);
-    }
+    case LIM_MC: return mc_of(m, r);
     case LIM_KOREN: {
       T a = m.template by<3>(T(1) + T(2) * r);
       T b = mmin(a, T(2));
@@ -116,10 +136,10 @@ __device__ __forceinline__ void muscl_face(M &m, int lim, T wi, T wip, T dA, T d
   }
   T r = limiter_ratio<T>(m, lim, dB, dA + E);
   T phi = slope_limiter<T>(m, lim, r, etaL);
-  left = wi + T(0.5) * phi * dA;
+  left = wi + m.half(phi) * dA;
   r = limiter_ratio<T>(m, lim, dB, dC + E);
   phi = slope_limiter<T>(m, lim, r, etaR);
-  right = wip - T(0.5) * phi * dC;
+  right = wip - m.half(phi) * dC;
 }
 
 // WENO2D_primvar.cpp:43-87: the two WENO3 face values of a cell with
@@ -129,7 +149,7 @@ template <typename T, class M>
 __device__ __forceinline__ void weno3_cell(M &m, T wm, T w, T wp, T &vL, T &vR) {
   const T e = eps_of<T>();
   {
-    T p0n = T(0.5) * wm + T(0.5) * w, p1n = T(1.5) * w - T(0.5) * wp;
+    T p0n = m.half(wm) + m.half(w), p1n = T(1.5) * w - m.half(wp);
     T B0n = (w - wm) * (w - wm), B1n = (wp - w) * (wp - w);
     T d0n = T(2.) / T(3.), d1n = T(1.) / T(3.);
     T a0n = m.div(d0n, (e + B0n) * (e + B0n)), a1n = m.div(d1n, (e + B1n) * (e + B1n));
@@ -138,7 +158,7 @@ __device__ __forceinline__ void weno3_cell(M &m, T wm, T w, T wp, T &vL, T &vR) 
     vR = w0n * p0n + w1n * p1n;
   }
   {
-    T p0p = T(1.5) * w - T(0.5) * wm, p1p = T(0.5) * wp + T(0.5) * w;
+    T p0p = T(1.5) * w - m.half(wm), p1p = m.half(wp) + m.half(w);
     T B0p = (w - wm) * (w - wm), B1p = (wp - w) * (wp - w);
     T d0p = T(1.) / T(3.), d1p = T(2.) / T(3.);
     T a0p = m.div(d0p, (e + B0p) * (e + B0p)), a1p = m.div(d1p, (e + B1p) * (e + B1p));
@@ -153,33 +173,33 @@ __device__ __forceinline__ void weno3_cell(M &m, T wm, T w, T wp, T &vL, T &vR) 
 template <typename T, bool RIGHT, class M>
 __device__ __forceinline__ T weno5_cell(M &m, T wmm, T wm, T w, T wp, T wpp) {
   const T e = eps_of<T>();
-  const T c13 = T(13.) / T(12.), c14 = T(1.) / T(4.);
+  const T c13 = T(13.) / T(12.);
   T t, t2;
   if (RIGHT) {
-    T p0n = m.template by<6>(T(-1) * wmm + T(5) * wm + T(2) * w);
-    T p1n = m.template by<6>(T(2) * wm + T(5) * w - wp);
-    T p2n = m.template by<6>(T(11) * w - T(7) * wp + T(2) * wpp);
-    t = wmm - T(2) * wm + w; t2 = wmm - T(4) * wm + T(3) * w;
-    T B0 = c13 * (t * t) + c14 * (t2 * t2);
-    t = wmm - T(2) * w + wp; t2 = wm - wp;
-    T B1 = c13 * (t * t) + c14 * (t2 * t2);
-    t = w - T(2) * wp + wpp; t2 = T(3) * w - T(4) * wp + wpp;
-    T B2 = c13 * (t * t) + c14 * (t2 * t2);
+    T p0n = m.template by<6>(-wmm + T(5) * wm + m.twice(w));
+    T p1n = m.template by<6>(m.twice(wm) + T(5) * w - wp);
+    T p2n = m.template by<6>(T(11) * w - T(7) * wp + m.twice(wpp));
+    t = wmm - m.twice(wm) + w; t2 = wmm - m.quad(wm) + T(3) * w;
+    T B0 = c13 * (t * t) + m.quarter(t2 * t2);
+    t = wmm - m.twice(w) + wp; t2 = wm - wp;
+    T B1 = c13 * (t * t) + m.quarter(t2 * t2);
+    t = w - m.twice(wp) + wpp; t2 = T(3) * w - m.quad(wp) + wpp;
+    T B2 = c13 * (t * t) + m.quarter(t2 * t2);
     T d0 = T(1.) / T(10.), d1 = T(6.) / T(10.), d2 = T(3.) / T(10.);
     T a0 = m.div(d0, (e + B0) * (e + B0)), a1 = m.div(d1, (e + B1) * (e + B1)), a2 = m.div(d2, (e + B2) * (e + B2));
     T as = a0 + a1 + a2;
     T w0 = m.div(a0, as), w1 = m.div(a1, as), w2 = m.div(a2, as);
     return w0 * p0n + w1 * p1n + w2 * p2n;
   } else {
-    T p0p = m.template by<6>(T(2) * wmm - T(7) * wm + T(11) * w);
-    T p1p = m.template by<6>(T(-1) * wm + T(5) * w + T(2) * wp);
-    T p2p = m.template by<6>(T(2) * w + T(5) * wp - wpp);
-    t = wmm - T(2) * wm + w; t2 = wmm - T(4) * wm + T(3) * w;
-    T B0 = c13 * (t * t) + c14 * (t2 * t2);
-    t = wmm - T(2) * w + wp; t2 = wm - wp;
-    T B1 = c13 * (t * t) + c14 * (t2 * t2);
-    t = w - T(2) * wp + wpp; t2 = T(3) * w - T(4) * wp + wpp;
-    T B2 = c13 * (t * t) + c14 * (t2 * t2);
+    T p0p = m.template by<6>(m.twice(wmm) - T(7) * wm + T(11) * w);
+    T p1p = m.template by<6>(-wm + T(5) * w + m.twice(wp));
+    T p2p = m.template by<6>(m.twice(w) + T(5) * wp - wpp);
+    t = wmm - m.twice(wm) + w; t2 = wmm - m.quad(wm) + T(3) * w;
+    T B0 = c13 * (t * t) + m.quarter(t2 * t2);
+    t = wmm - m.twice(w) + wp; t2 = wm - wp;
+    T B1 = c13 * (t * t) + m.quarter(t2 * t2);
+    t = w - m.twice(wp) + wpp; t2 = T(3) * w - m.quad(wp) + wpp;
+    T B2 = c13 * (t * t) + m.quarter(t2 * t2);
     T d0 = T(3.) / T(10.), d1 = T(6.) / T(10.), d2 = T(1.) / T(10.);
     T a0 = m.div(d0, (e + B0) * (e + B0)), a1 = m.div(d1, (e + B1) * (e + B1)), a2 = m.div(d2, (e + B2) * (e + B2));
     T as = a0 + a1 + a2;
@@ -196,7 +216,7 @@ __device__ __forceinline__ T fast_speed(M &m, const T *w, T gamma, int norm) {
   T can = m.root(m.div(w[norm] * w[norm], w[0]));
   T i0 = (ca * ca) + (a * a);
   T i1 = (ca * ca) - (a * a);
-  return m.root(T(0.5) * (i0 + m.root(i1 * i1 + T(4.) * (a * a) * ((ca * ca) - (can * can)))));
+  return m.root(m.half(i0 + m.root(i1 * i1 + m.quad(a * a) * ((ca * ca) - (can * can)))));
 }
 
 // the same for norm 5 (x) and 6 (y), whose first two terms are the same values
@@ -208,40 +228,53 @@ __device__ __forceinline__ void fast_speeds(M &m, const T *w, T gamma, T *cf) {
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const T can = m.root(m.div(w[5 + q] * w[5 + q], w[0]));
-    cf[q] = m.root(T(0.5) * (i0 + m.root(i1 * i1 + T(4.) * (a * a) * ((ca * ca) - (can * can)))));
+    cf[q] = m.root(m.half(i0 + m.root(i1 * i1 + m.quad(a * a) * ((ca * ca) - (can * can)))));
   }
 }
 
-// conserved state, physical flux, enthalpy, total pressure and energy of one
-// side (riemannS.cpp:59-108)
+// riemannS.cpp:59-108 for one side: the energy, the total pressure and the
+// fast speed; then, from those, the enthalpy, conserved state and physical flux
 template <typename T>
 struct Side {
   T q[8], F[8], H, pt, cf, e;
 };
 
 template <typename T, class M>
-__device__ __forceinline__ void side_state(M &m, const T *w, T gamma, Side<T> &s) {
-  s.cf = fast_speed<T>(m, w, gamma, 5);
-  const T vn = w[1], Bn = w[5];
-  T e = m.div(w[4], w[0] * (gamma - T(1))) + T(0.5) * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) +
-        m.div(T(0.5) * (w[5] * w[5] + w[6] * w[6] + w[7] * w[7]), w[0]);
+__device__ __forceinline__ void side_scalars(M &m, const T *w, T gamma, T &cf, T &pt, T &e) {
+  cf = fast_speed<T>(m, w, gamma, 5);
+  const T b2 = w[5] * w[5] + w[6] * w[6] + w[7] * w[7];
+  // the reference's 0.5*b2/rho: halving is exact, so it is half of the b2/rho
+  // the fast speed has
+  e = m.div(w[4], w[0] * (gamma - T(1))) + m.half(w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) + m.half(m.div(b2, w[0]));
   e = e * w[0];
-  s.e = e;
-  s.H = m.div(e + w[4] + T(0.5) * (w[5] * w[5] + w[6] * w[6] + w[7] * w[7]), w[0]);
-#pragma unroll
-  for (int k = 0; k < 8; k++) s.q[k] = w[k];
-  s.q[1] = w[0] * w[1]; s.q[2] = w[0] * w[2]; s.q[3] = w[0] * w[3];
-  s.q[4] = e;
-  const T pt = w[4] + T(0.5) * (w[5] * w[5] + w[6] * w[6] + w[7] * w[7]);
-  s.pt = pt;
-  s.F[0] = w[0] * vn;
-  s.F[1] = w[0] * vn * w[1] + pt - Bn * w[5];
-  s.F[2] = w[0] * vn * w[2] - Bn * w[6];
-  s.F[3] = w[0] * vn * w[3] - Bn * w[7];
-  s.F[4] = w[0] * vn * s.H - Bn * (w[1] * w[5] + w[2] * w[6] + w[3] * w[7]);
-  s.F[5] = vn * w[5] - Bn * w[1];
-  s.F[6] = vn * w[6] - Bn * w[2];
-  s.F[7] = vn * w[7] - Bn * w[3];
+  pt = w[4] + m.half(b2);
+}
+
+template <typename T, class M>
+__device__ __forceinline__ T enthalpy(M &m, const T *w, T e) {
+  return m.div(e + w[4] + m.half(w[5] * w[5] + w[6] * w[6] + w[7] * w[7]), w[0]);
+}
+
+template <typename T>
+__device__ __forceinline__ void side_flux(const T *w, T pt, T e, T H, T *q, T *F) {
+  const T vn = w[1], Bn = w[5];
+  q[0] = w[0]; q[1] = w[0] * w[1]; q[2] = w[0] * w[2]; q[3] = w[0] * w[3];
+  q[4] = e; q[5] = w[5]; q[6] = w[6]; q[7] = w[7];
+  F[0] = w[0] * vn;
+  F[1] = w[0] * vn * w[1] + pt - Bn * w[5];
+  F[2] = w[0] * vn * w[2] - Bn * w[6];
+  F[3] = w[0] * vn * w[3] - Bn * w[7];
+  F[4] = w[0] * vn * H - Bn * (w[1] * w[5] + w[2] * w[6] + w[3] * w[7]);
+  F[5] = vn * w[5] - Bn * w[1];
+  F[6] = vn * w[6] - Bn * w[2];
+  F[7] = vn * w[7] - Bn * w[3];
+}
+
+template <typename T, class M>
+__device__ __forceinline__ void side_state(M &m, const T *w, T gamma, Side<T> &s) {
+  side_scalars<T>(m, w, gamma, s.cf, s.pt, s.e);
+  s.H = enthalpy<T>(m, w, s.e);
+  side_flux<T>(w, s.pt, s.e, s.H, s.q, s.F);
 }
 
 // misc.cpp:95-140 Roe averages (sqrt(rhoL + sqrt(rhoR)) denominator as in
@@ -288,9 +321,9 @@ __device__ __forceinline__ int flux_rusa(M &m, const T *wL, const T *wR, T gamma
   side_state<T>(m, wL, gamma, L);
   side_state<T>(m, wR, gamma, R);
   const T a = L.cf + fabs(wL[1]), b = R.cf + fabs(wR[1]);
-  const T im = smax(a, b);
+  const T im = m.std_most(a, b);
 #pragma unroll
-  for (int k = 0; k < 8; k++) f[k] = T(0.5) * (L.F[k] + R.F[k]) - T(0.5) * im * (R.q[k] - L.q[k]);
+  for (int k = 0; k < 8; k++) f[k] = m.half(L.F[k] + R.F[k]) - m.half(im) * (R.q[k] - L.q[k]);
   return 0;
 }
 
@@ -361,96 +394,90 @@ __device__ __forceinline__ T dot13_57(T a1, T a2, T a3, T a5, T a6, T a7) {  // 
   return s;
 }
 
-// riemannS.cpp:397-549 (Miyoshi & Kusano).  Only the branch the wave fan
-// selects is assembled; its arithmetic is that of the reference.
+// riemannS.cpp:397-549 (Miyoshi & Kusano).  The wave fan selects one of six
+// regions; both star states and the waves are evaluated, then one side's
+// state, flux and star state are picked and the region's flux assembled once,
+// with the reference's operations in the reference's order.  (Evaluating
+// every region a warp's faces fall into, as a switch over them does, and both
+// sides' fluxes takes 40 % more FP64 instructions on the rotor.)
 template <typename T, class M>
 __device__ __forceinline__ int flux_hlld(M &m, const T *wL, const T *wR, T gamma, T *f) {
-  Side<T> L, R;
-  side_state<T>(m, wL, gamma, L);
-  side_state<T>(m, wR, gamma, R);
-  const T vnL = wL[1], vnR = wR[1], ptL = L.pt, ptR = R.pt;
-  const T SL = smin(vnL, vnR) - smax(L.cf, R.cf);
-  const T SR = smax(vnL, vnR) + smax(L.cf, R.cf);
-  const T SM = m.div((SR - vnR) * wR[0] * vnR - (SL - vnL) * wL[0] * vnL - ptR + ptL,
-                     (SR - vnR) * wR[0] - (SL - vnL) * wL[0]);
-  const T pts = m.div((SR - vnR) * wR[0] * ptL - (SL - vnL) * wL[0] * ptR +
-                          wL[0] * wR[0] * (SR - vnR) * (SL - vnL) * (vnR - vnL),
-                      (SR - vnR) * wR[0] - (SL - vnL) * wL[0]);
-  // left * state (:467-481)
-  const T rLs = m.div(wL[0] * (SL - vnL), SL - SM);
-  T vLs, wzLs, byLs, bzLs;
-  if ((wL[0] * (SL - wL[1]) * (SL - SM) - wL[5] * wL[5]) != T(0)) {
-    const T den = wL[0] * (SL - wL[1]) * (SL - SM) - wL[5] * wL[5];
-    vLs = wL[2] - wL[5] * wL[6] * m.div(SM - wL[1], den);
-    wzLs = wL[3] - wL[5] * wL[7] * m.div(SM - wL[1], den);
-    byLs = wL[6] * m.div(wL[0] * ((SL - wL[1]) * (SL - wL[1])) - wL[5] * wL[5], den);
-    bzLs = wL[7] * m.div(wL[0] * ((SL - wL[1]) * (SL - wL[1])) - wL[5] * wL[5], den);
-  } else {
-    vLs = wL[2]; wzLs = wL[3]; byLs = T(0.); bzLs = T(0.);
-  }
-  const T eLs = m.div((SL - wL[1]) * L.e - ptL * wL[1] + pts * SM +
-                          wL[5] * (dot13_57(wL[1], wL[2], wL[3], wL[5], wL[6], wL[7]) -
-                                   dot13_57(SM, vLs, wzLs, wL[5], byLs, bzLs)),
-                      SL - SM);
-  // right * state (:483-497)
-  const T rRs = m.div(wR[0] * (SR - vnR), SR - SM);
-  T vRs, wzRs, byRs, bzRs;
-  if ((wR[0] * (SR - wR[1]) * (SR - SM) - wR[5] * wR[5]) != T(0)) {
-    const T den = wR[0] * (SR - wR[1]) * (SR - SM) - wR[5] * wR[5];
-    vRs = wR[2] - wR[5] * wR[6] * m.div(SM - wR[1], den);
-    wzRs = wR[3] - wR[5] * wR[7] * m.div(SM - wR[1], den);
-    byRs = wR[6] * m.div(wR[0] * ((SR - wR[1]) * (SR - wR[1])) - wR[5] * wR[5], den);
-    bzRs = wR[7] * m.div(wR[0] * ((SR - wR[1]) * (SR - wR[1])) - wR[5] * wR[5], den);
-  } else {
-    vRs = wR[2]; wzRs = wR[3]; byRs = T(0); bzRs = T(0);
-  }
-  const T eRs = m.div((SR - wR[1]) * R.e - ptR * wR[1] + pts * SM +
-                          wR[5] * (dot13_57(wR[1], wR[2], wR[3], wR[5], wR[6], wR[7]) -
-                                   dot13_57(SM, vRs, wzRs, wR[5], byRs, bzRs)),
-                      SR - SM);
+  T cfL, ptL, eL, cfR, ptR, eR;
+  side_scalars<T>(m, wL, gamma, cfL, ptL, eL);
+  side_scalars<T>(m, wR, gamma, cfR, ptR, eR);
+  const T vnL = wL[1], vnR = wR[1];
+  const T cf = m.std_most(cfL, cfR);
+  const T SL = smin(vnL, vnR) - cf;
+  const T SR = smax(vnL, vnR) + cf;
+  const T mL = (SL - vnL) * wL[0], mR = (SR - vnR) * wR[0];
+  const T SM = m.div(mR * vnR - mL * vnL - ptR + ptL, mR - mL);
+  const T pts = m.div(mR * ptL - mL * ptR + wL[0] * wR[0] * (SR - vnR) * (SL - vnL) * (vnR - vnL), mR - mL);
+  // left and right * states (:467-497)
+  auto star = [&](const T *w, T S, T e, T pt, T ms, T &r, T &v, T &wz, T &by, T &bz, T &d, T &es) {
+    r = m.div(ms, S - SM);   // w0 * (S - vn) is (S - vn) * w0
+    const T den = ms * (S - SM) - w[5] * w[5];
+    if (m.nonzero(den)) {
+      const T k = m.div(SM - w[1], den);
+      const T h = m.div(w[0] * ((S - w[1]) * (S - w[1])) - w[5] * w[5], den);
+      v = w[2] - w[5] * w[6] * k;
+      wz = w[3] - w[5] * w[7] * k;
+      by = w[6] * h;
+      bz = w[7] * h;
+    } else {
+      v = w[2]; wz = w[3]; by = T(0.); bz = T(0.);
+    }
+    d = dot13_57(SM, v, wz, w[5], by, bz);
+    es = m.div((S - w[1]) * e - pt * w[1] + pts * SM +
+                   w[5] * (dot13_57(w[1], w[2], w[3], w[5], w[6], w[7]) - d),
+               S - SM);
+  };
+  T rLs, vLs, wzLs, byLs, bzLs, dLs, eLs, rRs, vRs, wzRs, byRs, bzRs, dRs, eRs;
+  star(wL, SL, eL, ptL, mL, rLs, vLs, wzLs, byLs, bzLs, dLs, eLs);
+  star(wR, SR, eR, ptR, mR, rRs, vRs, wzRs, byRs, bzRs, dRs, eRs);
   const T sLs = m.root(rLs), sRs = m.root(rRs);
   const T SLs = SM - m.div(fabs(wL[5]), sLs);
   const T SRs = SM + m.div(fabs(wR[5]), sRs);
   int br = -1;
-  if (SL > T(0)) br = 0;
-  else if (SL <= T(0.) && SLs >= T(0.)) br = 1;
-  else if (SLs <= T(0.) && SM >= T(0.)) br = 2;
-  else if (SM <= T(0.) && SRs >= T(0.)) br = 3;
-  else if (SRs <= T(0.) && SR >= T(0.)) br = 4;
-  else if (SR < T(0.)) br = 5;
-  // conserved * states (w2u, misc.cpp:82-92; energy replaced, :524,527)
-  const T qLs[8] = {rLs, rLs * SM, rLs * vLs, rLs * wzLs, eLs, wL[5], byLs, bzLs};
-  const T qRs[8] = {rRs, rRs * SM, rRs * vRs, rRs * wzRs, eRs, wR[5], byRs, bzRs};
-  T qss[8];
-  if (br == 2 || br == 3) {
-    // ** states (:501-519); the right ** state is a copy of the left one (:517)
-    const T sg = sgn(wL[5]);
-    const T vss = m.div(sLs * vLs + sRs * vRs + (byRs - byLs) * sg, sLs + sRs);
-    const T wss = m.div(sLs * wzLs + sRs * wzRs + (bzRs - bzLs) * sg, sLs + sRs);
-    const T byss = m.div(sLs * byRs + sRs * byLs + m.root(rLs * rRs) * (vRs - vLs) * sg, sLs + sRs);
-    const T bzss = m.div(sLs * bzRs + sRs * bzLs + m.root(rLs * rRs) * (wzRs - wzLs) * sg, sLs + sRs);
+  if (m.positive(SL)) br = 0;
+  else if (m.nonpositive(SL) && m.nonnegative(SLs)) br = 1;
+  else if (m.nonpositive(SLs) && m.nonnegative(SM)) br = 2;
+  else if (m.nonpositive(SM) && m.nonnegative(SRs)) br = 3;
+  else if (m.nonpositive(SRs) && m.nonnegative(SR)) br = 4;
+  else if (m.negative(SR)) br = 5;
+  const bool left = br <= 2, mid = br == 2 || br == 3, fan = mid || br == 1 || br == 4;
+  // the picked side: its state, flux, star state and waves
+  T w[8], q[8], F[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) w[k] = left ? wL[k] : wR[k];
+  const T e = left ? eL : eR;
+  side_flux<T>(w, left ? ptL : ptR, e, enthalpy<T>(m, w, e), q, F);
+  const T S = left ? SL : SR, Ss = left ? SLs : SRs, ss = left ? sLs : sRs;
+  const T rs = left ? rLs : rRs, es = left ? eLs : eRs;
+  const T vs = left ? vLs : vRs, wzs = left ? wzLs : wzRs, bys = left ? byLs : byRs, bzs = left ? bzLs : bzRs;
+  // conserved * state (w2u, misc.cpp:82-92; energy replaced, :524,527)
+  const T qs[8] = {rs, rs * SM, rs * vs, rs * wzs, es, w[5], bys, bzs};
+  T x[8];   // the state the wave Sx multiplies: the ** state (:501-519) or the * state
+  T Sx = S;
+#pragma unroll
+  for (int k = 0; k < 8; k++) x[k] = qs[k];
+  if (mid) {  // the right ** state is a copy of the left one (:517)
+    const T sg = sgn(wL[5]), sum = sLs + sRs, rr = m.root(rLs * rRs);
+    const T vss = m.div(sLs * vLs + sRs * vRs + (byRs - byLs) * sg, sum);
+    const T wss = m.div(sLs * wzLs + sRs * wzRs + (bzRs - bzLs) * sg, sum);
+    const T byss = m.div(sLs * byRs + sRs * byLs + rr * (vRs - vLs) * sg, sum);
+    const T bzss = m.div(sLs * bzRs + sRs * bzLs + rr * (wzRs - wzLs) * sg, sum);
     const T dss = dot13_57(SM, vss, wss, wL[5], byss, bzss);
-    T ess;
-    if (br == 2)
-      ess = eLs - sLs * (dot13_57(SM, vLs, wzLs, wL[5], byLs, bzLs) - dss) * sg;
-    else
-      ess = eRs + sRs * (dot13_57(SM, vRs, wzRs, wR[5], byRs, bzRs) - dss) * sgn(wR[5]);
-    qss[0] = rLs; qss[1] = rLs * SM; qss[2] = rLs * vss; qss[3] = rLs * wss;
-    qss[4] = ess; qss[5] = wL[5]; qss[6] = byss; qss[7] = bzss;
+    const T de = ss * ((left ? dLs : dRs) - dss) * (left ? sg : sgn(wR[5]));
+    x[0] = rLs; x[1] = rLs * SM; x[2] = rLs * vss; x[3] = rLs * wss;
+    x[4] = es + (left ? -de : de); x[5] = wL[5]; x[6] = byss; x[7] = bzss;
+    Sx = Ss;
   }
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    T v = T(0);
-    switch (br) {
-      case 0: v = L.F[k]; break;
-      case 1: v = L.F[k] + SL * qLs[k] - SL * L.q[k]; break;
-      case 2: v = L.F[k] + SLs * qss[k] - (SLs - SL) * qLs[k] - SL * L.q[k]; break;
-      case 3: v = R.F[k] + SRs * qss[k] - (SRs - SR) * qRs[k] - SR * R.q[k]; break;
-      case 4: v = R.F[k] + SR * qRs[k] - SR * R.q[k]; break;
-      case 5: v = R.F[k]; break;
-      default: break;
-    }
-    f[k] = v;
+    T v = F[k] + Sx * x[k];
+    const T v2 = v - (Ss - S) * qs[k];
+    v = (mid ? v2 : v) - S * q[k];
+    f[k] = fan ? v : (br < 0 ? T(0) : F[k]);
   }
   return 0;
 }

@@ -10,9 +10,10 @@
 // as IEEE division and square root in round to nearest even.  Measured on one
 // GB300, 12 warps per SM: 26 clocks per SM and warp for an addition and a
 // division (115 with the compiler's), 25 for an addition and a square root
-// (115).  The face kernel of a 196-block rotor (MC + HLLD): 257 -> 172 us
-// and 3.57 -> 2.06 M FP64-pipe instructions; of the 256-block KH layer (MC +
-// RUSA): 207 -> 144 us.
+// (115).  The face kernel with the Soft arithmetic, 196-block rotor (MC +
+// HLLD): 257 -> 100 us and 3.57 -> 1.43 M FP64-pipe instructions; 256-block KH
+// layer (MC + RUSA): 207 -> 92 us; 256-block Orszag-Tang (WENO5 + HLLD): 790
+// -> 300 us.
 //
 // Method (long division with a large radix, two digits; e.g. Ercegovac &
 // Lang, Digital Arithmetic, ch. 5 and 7): a 23-bit reciprocal from MUFU,
@@ -232,9 +233,24 @@ AMR_HD double sqrt_rn(double x, bool &bad) {
   return zero ? x : bits_f64(hi, static_cast<uint32_t>(n));
 }
 
+// 2^K x, exact: the exponent field moved, zeros kept.  A result or operand
+// outside the normal range sets `bad`.
+template <int K>
+AMR_HD double scale_pow2(double x, bool &bad) {
+  const uint64_t u = f64_bits(x);
+  const uint32_t h = static_cast<uint32_t>(u >> 32), l = static_cast<uint32_t>(u);
+  const uint32_t t = h << 1;
+  const bool zero = (t | l) == 0u;
+  constexpr uint32_t down = K < 0 ? -K : 0, up = K > 0 ? K : 0;
+  bad |= !(zero || t - ((1u + down) << 21) < ((2046u - up - down) << 21));
+  return bits_f64(zero ? h : h + (static_cast<uint32_t>(K) << 20), l);
+}
+
 #ifdef __CUDACC__
 // The arithmetic a formula is evaluated with: the operators of the type, or,
-// for double, the routines above.  After a Soft evaluation that reports
+// for double, the routines above and comparisons and multiplications by
+// powers of two on the bit patterns (3 to 7 integer instructions each, where
+// the FP64 pipe takes 16 clocks per warp).  After a Soft evaluation that reports
 // failed(), some operand was outside the routines' range and the results are
 // meaningless: evaluate again with Native.
 template <typename T>
@@ -245,6 +261,19 @@ struct Native {
   // the larger of two values that are not negative; Soft compares the bits,
   // where a NaN counts as the largest (and the division it reaches fails)
   __device__ __forceinline__ T most(T a, T b) { return a > b ? a : b; }
+  __device__ __forceinline__ T std_most(T a, T b) { return a < b ? b : a; }   // std::max, for a NaN in b
+  __device__ __forceinline__ T least(T a, T b) { return a < b ? a : b; }
+  // multiplications by powers of two
+  __device__ __forceinline__ T half(T a) { return T(0.5) * a; }
+  __device__ __forceinline__ T quarter(T a) { return T(0.25) * a; }
+  __device__ __forceinline__ T twice(T a) { return T(2) * a; }
+  __device__ __forceinline__ T quad(T a) { return T(4) * a; }
+  // comparisons with zero
+  __device__ __forceinline__ bool positive(T a) { return a > T(0); }
+  __device__ __forceinline__ bool negative(T a) { return a < T(0); }
+  __device__ __forceinline__ bool nonpositive(T a) { return a <= T(0); }
+  __device__ __forceinline__ bool nonnegative(T a) { return a >= T(0); }
+  __device__ __forceinline__ bool nonzero(T a) { return a != T(0); }
   __device__ __forceinline__ bool failed() const { return false; }
 };
 struct Soft {
@@ -253,6 +282,18 @@ struct Soft {
   __device__ __forceinline__ double root(double x) { return sqrt_rn(x, bad); }
   template <int B> __device__ __forceinline__ double by(double a) { return div_by<B>(a, bad); }
   __device__ __forceinline__ double most(double a, double b) { return f64_bits(a) > f64_bits(b) ? a : b; }
+  __device__ __forceinline__ double std_most(double a, double b) { return most(a, b); }
+  __device__ __forceinline__ double least(double a, double b) { return f64_bits(a) < f64_bits(b) ? a : b; }
+  __device__ __forceinline__ double half(double a) { return scale_pow2<-1>(a, bad); }
+  __device__ __forceinline__ double quarter(double a) { return scale_pow2<-2>(a, bad); }
+  __device__ __forceinline__ double twice(double a) { return scale_pow2<1>(a, bad); }
+  __device__ __forceinline__ double quad(double a) { return scale_pow2<2>(a, bad); }
+  // of numbers (a NaN fails in the divisions around them)
+  __device__ __forceinline__ bool positive(double a) { return __double_as_longlong(a) > 0; }
+  __device__ __forceinline__ bool negative(double a) { return __double_as_longlong(a) < 0 && nonzero(a); }
+  __device__ __forceinline__ bool nonpositive(double a) { return !positive(a); }
+  __device__ __forceinline__ bool nonnegative(double a) { return !negative(a); }
+  __device__ __forceinline__ bool nonzero(double a) { return (f64_bits(a) << 1) != 0; }
   __device__ __forceinline__ bool failed() const { return bad; }
 };
 template <typename T> struct ArithOf { using type = Native<T>; };

@@ -213,19 +213,27 @@ __device__ __forceinline__ bool bulk_stage_wait(uint64_t *bar, uint32_t phase) {
   return false;
 }
 
+// plane of variable k of the face frame (normal, tangential, z): riemannS
+// rotates a y face (riemannS.cpp:12-23, 47-55), u <-> v and Bx <-> By
+__device__ __forceinline__ int face_plane(int k, bool yf) {
+  const int r = k == 1 ? 2 : k == 2 ? 1 : k == 5 ? 6 : k == 6 ? 5 : k;
+  return yf ? r : k;
+}
+
 // MUSCL2D.cpp:24-116 for one face: W is plane 0 of the block's primitive
 // state (planes NN apart), cL the cell on its left (below it), s the cell
 // stride along its normal, yf whether that is y; bn the face's own normal
-// field (the CT override, MUSCL2D.cpp:48-51).  Returns riemann()'s code.
+// field (the CT override, MUSCL2D.cpp:48-51).  The states are read and the
+// flux is returned in the face frame, so that x and y faces of a warp run
+// the same code.  Returns riemann()'s code.
 template <int RECON, int FLUX, int NN, typename T, class M>
 __device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma,
                                             T *fl) {
-  const int kn = yf ? 6 : 5;                                // normal B component
   T wl[8], wr[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    if (k == kn) continue;
-    const T *w = W + k * NN + cL;
+    if (k == 5) continue;
+    const T *w = W + face_plane(k, yf) * NN + cL;
     if (RECON == REC_MUSCL) {
       const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
       muscl_face<T>(m, lim, w0, w1, w0 - wm, w1 - w0, w2 - w1, h, wl[k], wr[k]);
@@ -238,32 +246,21 @@ __device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, boo
       wr[k] = weno5_cell<T, true>(m, w[-s], w[0], w[s], w[2 * s], w[3 * s]);
     }
   }
-  wl[kn] = bn;
-  wr[kn] = bn;
-  if (!yf) return riemann<FLUX, T>(m, wl, wr, gamma, fl);
-  // riemannS.cpp:12-23, 47-55: rotate y into x and back
-  T l2[8], r2[8], f2[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) { l2[k] = wl[k]; r2[k] = wr[k]; }
-  l2[1] = wl[2]; l2[2] = wl[1]; r2[1] = wr[2]; r2[2] = wr[1];
-  l2[5] = wl[6]; l2[6] = wl[5]; r2[5] = wr[6]; r2[6] = wr[5];
-  const int rc = riemann<FLUX, T>(m, l2, r2, gamma, f2);
-#pragma unroll
-  for (int k = 0; k < 8; k++) fl[k] = f2[k];
-  fl[1] = f2[2]; fl[2] = f2[1]; fl[5] = f2[6]; fl[6] = f2[5];
-  return rc;
+  wl[5] = bn;
+  wr[5] = bn;
+  return riemann<FLUX, T>(m, wl, wr, gamma, fl);
 }
 
 // the same with the native operators, for the rare face whose operands left
 // the range of the Soft arithmetic; a function of its own, so that its
-// registers are not the hot path's.  The flux goes to out[k * NN].
+// registers are not the hot path's.  The flux goes to its planes of `out`.
 template <int RECON, int FLUX, int NN, typename T>
 __device__ __noinline__ int face_flux_native(const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma, T *out) {
   Native<T> m;
   T fl[8];
   const int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, lim, h, bn, gamma, fl);
 #pragma unroll
-  for (int k = 0; k < 8; k++) out[k * NN] = fl[k];
+  for (int k = 0; k < 8; k++) out[face_plane(k, yf) * NN] = fl[k];
   return rc;
 }
 
@@ -367,20 +364,17 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
       T *out = (yf ? gg : ff) + fpos;
       rc = face_flux_native<RECON, FLUX, NN, T>(sW, cL, s, yf, lim, h, bn, gamma, out);
 #pragma unroll
-      for (int k = 0; k < 8; k++) fl[k] = out[k * NN];
+      for (int k = 0; k < 8; k++) fl[k] = out[face_plane(k, yf) * NN];
     }
     if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
     bool bad = false;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       bad |= bits_nan(fl[k]);
-      if (!yf) {
-        sFx[(k * NF + r) * NFX + (c + 1)] = fl[k];
-        ff[k * NN + fpos] = fl[k];
-      } else {
-        sFy[(k * NFX + (r + 1)) * NF + c] = fl[k];
-        gg[k * NN + fpos] = fl[k];
-      }
+      const int p = face_plane(k, yf);
+      if (!yf) sFx[(p * NF + r) * NFX + (c + 1)] = fl[k];
+      else sFy[(p * NFX + (r + 1)) * NF + c] = fl[k];
+      (yf ? gg : ff)[p * NN + fpos] = fl[k];
     }
     if (bad) dev_fail(a.err, DERR_NAN, task.slot, fpos % N, fpos / N, 0.0);
   }

@@ -87,7 +87,10 @@ __global__ void __launch_bounds__(256) k_prim_task(SplitArgs a) {
 }
 
 // MUSCL2D.cpp:24-116 for one face of one leaf: x faces (i+1/2, j) for i, j in
-// [LO, HI], then y faces (i, j+1/2)
+// [LO, HI], then y faces (i, j+1/2).  On the FP64 path the kernels around it
+// are bound by the FP64 pipe (76-80 % busy with 12 warps per SM): about 230
+// FP64 instructions per MC + RUSA face and 330 per MC + HLLD face, all of them
+// additions and multiplications (softfp.cuh takes the rest).
 template <int NG, int RECON, int FLUX, typename S>
 __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
   using G = Geo<NG>;
@@ -114,14 +117,14 @@ __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
   if (m.failed()) {
     rc = face_flux_native<RECON, FLUX, NN, T>(W, cL, s, yf, ip.limiter, h, bn, gamma, out);
 #pragma unroll
-    for (int k = 0; k < 8; k++) fl[k] = out[k * NN];
+    for (int k = 0; k < 8; k++) fl[k] = out[face_plane(k, yf) * NN];
   }
   if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
   bool bad = false;
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     bad |= bits_nan(fl[k]);
-    out[k * NN] = fl[k];
+    out[face_plane(k, yf) * NN] = fl[k];
   }
   if (bad) dev_fail(a.err, DERR_NAN, task.slot, fpos % N, fpos / N, 0.0);
 }

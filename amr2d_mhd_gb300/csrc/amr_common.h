@@ -64,6 +64,7 @@ struct InstParams {
   double dt;      // dom.dt of the current step
   int limiter;
   int ct_type;    // 2 = upwind-switched EMF (CT2D.cpp:28-75), else the average
+  float gm1_hi, gm1_lo;   // gamma - 1 as a pair of floats (FP32 path)
 };
 
 // One gather of a compiled ghost fill (see ghost_compile.cpp).  The same op

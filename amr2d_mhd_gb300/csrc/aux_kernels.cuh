@@ -26,8 +26,9 @@ __global__ void k_ghost_snap(GhostLaunch g) {
   int q, k;
   const GhostSeg s = ghost_seg(g, blockIdx.y, q, k);
   const size_t at = (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos;
-  g.snapbuf[(static_cast<size_t>(q) * g.nsnaps + r) * 8 + k] =
-      s.f32 ? static_cast<double>(static_cast<const float *>(s.field)[at]) : static_cast<const double *>(s.field)[at];
+  const size_t to = static_cast<size_t>(r) * 8 + k;
+  if (s.f32) snap_rows<float>(g.snapbuf, q, g.nsnaps)[to] = static_cast<const float *>(s.field)[at];
+  else snap_rows<double>(g.snapbuf, q, g.nsnaps)[to] = static_cast<const double *>(s.field)[at];
 }
 
 template <int N>
@@ -39,9 +40,8 @@ __global__ void k_ghost_apply(GhostLaunch g) {
   if (op.type == GOP_NOP) return;  // padding of an instance's range
   int q, k;
   const GhostSeg s = ghost_seg(g, blockIdx.y, q, k);
-  const double *snap = g.snapbuf + static_cast<size_t>(q) * g.nsnaps * 8;
-  if (s.f32) ghost_apply_one<N, float>(s, op, k, snap);
-  else ghost_apply_one<N, double>(s, op, k, snap);
+  if (s.f32) ghost_apply_one<N, float>(s, op, k, snap_rows<float>(g.snapbuf, q, g.nsnaps));
+  else ghost_apply_one<N, double>(s, op, k, snap_rows<double>(g.snapbuf, q, g.nsnaps));
 }
 
 // ------------------------------------------------------------- CT2D.cpp
@@ -257,7 +257,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, DevError *err) {
 // of the fluxes and face field that precedes CT2D (main.cpp:161-163), and
 // the cell phase saves the snapshots of the cell fill that follows it.
 template <int NG, typename S, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
+__global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1536 : 1024) / THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
                                                      unsigned *bar) {
   pdl_wait();
   constexpr int NN = Geo<NG>::NN;
@@ -314,7 +314,9 @@ __global__ void __launch_bounds__(128) k_diffuse(CtArgs a) {
 // the FP32 path computes the cell values in FP32 and reduces them in FP64).
 // The FP64 form was bound by the FP64 pipe; with divisions, roots and the
 // criterion's maxima on the integer pipe (softfp.cuh) it takes 25 us for the
-// 196 leaves of a rotor, 60 before.
+// 196 leaves of a rotor, 60 before.  The FP32 form was bound by the FP64
+// instructions of the pressure recovery (76 % busy); with pairs of floats
+// (cons2prim_cell) 85 us for 6272 leaves, 103 before.
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -346,8 +348,11 @@ struct DtArgs {
   FillFuse fuse;    // fused fills: the fill of U after the step, gathered first
 };
 
+// resident CTAs of k_dt_cell: the FP32 form has to hide its loads (32 registers)
+template <typename S> struct DtMinBlocks { static constexpr int value = 5; };
+template <> struct DtMinBlocks<float> { static constexpr int value = 8; };
 template <int NG, typename S>
-__global__ void __launch_bounds__(256) k_dt_cell(DtArgs a) {
+__global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a) {
   pdl_wait();
   using G = Geo<NG>;
   using T = S;
@@ -362,7 +367,7 @@ __global__ void __launch_bounds__(256) k_dt_cell(DtArgs a) {
     S u[8], w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = U[k * NN + c];
-    cons2prim_cell<S>(u, w, a.inst[t.inst].gamma);
+    cons2prim_cell<S>(u, w, GasGamma<S>(a.inst[t.inst]));
 #pragma unroll
     for (int k = 0; k < 8; k++) sW[k * NN + c] = w[k];
     const int i = c % N, j = c / N;
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(kRefineChunk) k_refine(TreeOpArgs a) {
     for (int k = 0; k < 8; k++) Sn[k * NN + c] = u[k];
     // U2W("refine") pressure trap (refine.cpp:70-82)
     T w[8];
-    cons2prim_cell<S>(u, w, a.inst[op.inst].gamma);
+    cons2prim_cell<S>(u, w, GasGamma<S>(a.inst[op.inst]));
     if (w[4] <= T(0) && i > G::LO && i < G::HI + 1 && j > G::LO && j < G::HI + 1)
       dev_fail(a.err, DERR_PRESSURE, op.son[sq], i, j, static_cast<double>(w[4]));
   }
@@ -772,7 +777,7 @@ __global__ void k_coarsen(TreeOpArgs a) {
     S u[8], w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = D[k * NN + c];
-    cons2prim_cell<S>(u, w, a.inst[op.inst].gamma);
+    cons2prim_cell<S>(u, w, GasGamma<S>(a.inst[op.inst]));
     const int i = c % N, j = c / N;
     if (w[4] <= S(0) && i > G::LO && i < G::HI + 1 && j > G::LO && j < G::HI + 1)
       dev_fail(a.err, DERR_PRESSURE, op.dad, i, j, static_cast<double>(w[4]));

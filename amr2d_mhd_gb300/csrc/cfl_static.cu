@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) k_cfl_static_blocks(const double *U, cons
     double u[8], w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = u0[k * NN + c];
-    cons2prim_cell<double>(u, w, gamma);
+    cons2prim_cell<double>(u, w, GasGamma<double>(gamma));
     double v1 = 0, v2 = 0;
     evaluate<double>([&](auto &ar) {
       double cf[2];

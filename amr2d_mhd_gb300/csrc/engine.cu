@@ -522,6 +522,8 @@ void Engine::fill_params_host() {
     p[q].dt = inst_[q].dt;
     p[q].limiter = inst_[q].limiter;
     p[q].ct_type = inst_[q].cfg.ct_type == 2 ? 2 : 1;
+    p[q].gm1_hi = static_cast<float>(inst_[q].gamma - 1);
+    p[q].gm1_lo = static_cast<float>((inst_[q].gamma - 1) - static_cast<double>(p[q].gm1_hi));
   }
 }
 

@@ -27,7 +27,7 @@ struct GhostLaunch {
   int nops, nsnaps;
   GhostSeg seg[kMaxSeg];
   int nseg;
-  double *snapbuf;    // [nseg][nsnaps][8]
+  double *snapbuf;    // [nseg][nsnaps][8], values of the segment's type (snap_rows)
   // variable rows of the launch: segment q owns rows [row0[q], row0[q+1]);
   // set by launch_ghost
   int row0[kMaxSeg + 1];
@@ -68,7 +68,7 @@ __device__ __forceinline__ F fine_value(int kind, int k, F a00, F a01, F a10, F 
 // not null, to the destination block's copy of the field in shared memory
 // ([nv][N*N])
 template <int N, typename F>
-__device__ __forceinline__ void ghost_gather(const GhostSeg &s, const GhostOp &op, int k, const double *snap, F &v0,
+__device__ __forceinline__ void ghost_gather(const GhostSeg &s, const GhostOp &op, int k, const F *snap, F &v0,
                                              F &v1) {
   constexpr int NN = N * N;
   const F *fld = static_cast<const F *>(s.field);
@@ -84,10 +84,8 @@ __device__ __forceinline__ void ghost_gather(const GhostSeg &s, const GhostOp &o
     const F *c = fld + (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos;
     v0 = op.type == GOP_COPY ? c[0] : fine_value<F>(s.kind, k, c[0], c[N], c[1], c[1 + N]);
   } else {
-    const double *r = snap + static_cast<size_t>(op.src_slot) * 8 + k;
-    v0 = op.type == GOP_SNAP ? static_cast<F>(r[0])
-                             : fine_value<F>(s.kind, k, static_cast<F>(r[0]), static_cast<F>(r[8]),
-                                             static_cast<F>(r[16]), static_cast<F>(r[24]));
+    const F *r = snap + static_cast<size_t>(op.src_slot) * 8 + k;
+    v0 = op.type == GOP_SNAP ? r[0] : fine_value<F>(s.kind, k, r[0], r[8], r[16], r[24]);
   }
 }
 
@@ -108,9 +106,17 @@ __device__ __forceinline__ void ghost_put(const GhostSeg &s, const GhostOp &op, 
   if (tile) tile[k * NN + op.dst_pos] = v0;
 }
 
+// A snapshot row holds 8 values of the field's own type (no conversion of
+// FP32 values to double and back on the FP64 pipe); segment q's rows start at
+// q * nsnaps rows of 8 doubles.
+template <typename F>
+__device__ __forceinline__ F *snap_rows(double *snapbuf, int q, int nsnaps) {
+  return reinterpret_cast<F *>(snapbuf + static_cast<size_t>(q) * nsnaps * 8);
+}
+
 // variable k of one gather (`tile` as for ghost_put)
 template <int N, typename F>
-__device__ __forceinline__ void ghost_apply_one(const GhostSeg &s, const GhostOp &op, int k, const double *snap,
+__device__ __forceinline__ void ghost_apply_one(const GhostSeg &s, const GhostOp &op, int k, const F *snap,
                                                 F *tile = nullptr) {
   F v0, v1 = F(0.);
   ghost_gather<N, F>(s, op, k, snap, v0, v1);
@@ -132,7 +138,7 @@ struct FillPass {
   int nseg;             // 0: no fill
   int rows;             // variables over the segments
   int tile_seg;         // segment mirrored in the consuming kernel's shared memory (-1: none)
-  double *snapbuf;      // [nseg][nsnaps][8]
+  double *snapbuf;      // [nseg][nsnaps][8], values of the segment's type (snap_rows)
 };
 struct FillFuse {
   const GhostOp *ops;
@@ -164,19 +170,21 @@ __device__ __forceinline__ void fill_apply_task(const FillFuse &f, const LeafTas
     const GhostOp op = f.ops[t.op_begin + (e - row * n)];
     int q, k;
     const GhostSeg s = pass_seg(f.apply, row, q, k);
-    const double *snap = f.apply.snapbuf + static_cast<size_t>(q) * f.nsnaps * 8;
     TileT *tl = q == f.apply.tile_seg ? tile : nullptr;
-    if (s.f32) ghost_apply_one<N, float>(s, op, k, snap, reinterpret_cast<float *>(tl));
-    else ghost_apply_one<N, double>(s, op, k, snap, reinterpret_cast<double *>(tl));
+    if (s.f32)
+      ghost_apply_one<N, float>(s, op, k, snap_rows<float>(f.apply.snapbuf, q, f.nsnaps), reinterpret_cast<float *>(tl));
+    else
+      ghost_apply_one<N, double>(s, op, k, snap_rows<double>(f.apply.snapbuf, q, f.nsnaps),
+                                 reinterpret_cast<double *>(tl));
   }
 }
 
 // The first gather of a thread, loaded ahead (while the fused stage
 // kernel's bulk copy is in flight) and stored by fill_apply_task_after; the
-// values are held as double (exact for float fields).
+// values are held as their bits (a float's in the low word).
 struct FillPre {
   GhostOp op;
-  double v0, v1;
+  long long v0, v1;
   int row;
   bool on;
 };
@@ -191,14 +199,16 @@ __device__ __forceinline__ FillPre fill_prefetch(const FillFuse &f, const LeafTa
   p.op = f.ops[t.op_begin + (tid - p.row * n)];
   int q, k;
   const GhostSeg s = pass_seg(f.apply, p.row, q, k);
-  const double *snap = f.apply.snapbuf + static_cast<size_t>(q) * f.nsnaps * 8;
   if (s.f32) {
     float a = 0.f, b = 0.f;
-    ghost_gather<N, float>(s, p.op, k, snap, a, b);
-    p.v0 = a;
-    p.v1 = b;
+    ghost_gather<N, float>(s, p.op, k, snap_rows<float>(f.apply.snapbuf, q, f.nsnaps), a, b);
+    p.v0 = __float_as_int(a);
+    p.v1 = __float_as_int(b);
   } else {
-    ghost_gather<N, double>(s, p.op, k, snap, p.v0, p.v1);
+    double a = 0., b = 0.;
+    ghost_gather<N, double>(s, p.op, k, snap_rows<double>(f.apply.snapbuf, q, f.nsnaps), a, b);
+    p.v0 = __double_as_longlong(a);
+    p.v1 = __double_as_longlong(b);
   }
   return p;
 }
@@ -212,10 +222,11 @@ __device__ __forceinline__ void fill_apply_task_after(const FillFuse &f, const L
     const GhostSeg s = pass_seg(f.apply, p.row, q, k);
     TileT *tl = q == f.apply.tile_seg ? tile : nullptr;
     if (s.f32)
-      ghost_put<N, float>(s, p.op, k, static_cast<float>(p.v0), static_cast<float>(p.v1),
+      ghost_put<N, float>(s, p.op, k, __int_as_float(static_cast<int>(p.v0)), __int_as_float(static_cast<int>(p.v1)),
                           reinterpret_cast<float *>(tl));
     else
-      ghost_put<N, double>(s, p.op, k, p.v0, p.v1, reinterpret_cast<double *>(tl));
+      ghost_put<N, double>(s, p.op, k, __longlong_as_double(p.v0), __longlong_as_double(p.v1),
+                           reinterpret_cast<double *>(tl));
   }
   const int n = t.op_count;
   const int total = n * f.apply.rows;
@@ -224,10 +235,12 @@ __device__ __forceinline__ void fill_apply_task_after(const FillFuse &f, const L
     const GhostOp op = f.ops[t.op_begin + (e - row * n)];
     int q, k;
     const GhostSeg s = pass_seg(f.apply, row, q, k);
-    const double *snap = f.apply.snapbuf + static_cast<size_t>(q) * f.nsnaps * 8;
     TileT *tl = q == f.apply.tile_seg ? tile : nullptr;
-    if (s.f32) ghost_apply_one<N, float>(s, op, k, snap, reinterpret_cast<float *>(tl));
-    else ghost_apply_one<N, double>(s, op, k, snap, reinterpret_cast<double *>(tl));
+    if (s.f32)
+      ghost_apply_one<N, float>(s, op, k, snap_rows<float>(f.apply.snapbuf, q, f.nsnaps), reinterpret_cast<float *>(tl));
+    else
+      ghost_apply_one<N, double>(s, op, k, snap_rows<double>(f.apply.snapbuf, q, f.nsnaps),
+                                 reinterpret_cast<double *>(tl));
   }
 }
 
@@ -235,8 +248,9 @@ __device__ __forceinline__ void snap_one(const FillFuse &f, int NN, const GhostS
   int q, k;
   const GhostSeg s = pass_seg(f.save, row, q, k);
   const size_t at = (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos;
-  f.save.snapbuf[(static_cast<size_t>(q) * f.nsnaps + r) * 8 + k] =
-      s.f32 ? static_cast<double>(static_cast<const float *>(s.field)[at]) : static_cast<const double *>(s.field)[at];
+  const size_t to = static_cast<size_t>(r) * 8 + k;
+  if (s.f32) snap_rows<float>(f.save.snapbuf, q, f.nsnaps)[to] = static_cast<const float *>(s.field)[at];
+  else snap_rows<double>(f.save.snapbuf, q, f.nsnaps)[to] = static_cast<const double *>(s.field)[at];
 }
 
 // the snapshots of the next fill (`f.save`) that lie in task t's block; the

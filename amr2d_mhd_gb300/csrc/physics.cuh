@@ -57,6 +57,11 @@ __device__ __forceinline__ double minmod_of(Soft &m, double r) {
   const double c = m.least(r, 1.0);
   return __double2hiint(r) < 0 ? (m.nonzero(r) ? 0.0 : r) : c;
 }
+// FP32 faces: single instructions for the comparisons
+__device__ __forceinline__ float minmod_of(Quick &, float r) { return fmaxf(0.f, fminf(1.f, r)); }
+__device__ __forceinline__ float mc_of(Quick &, float r) {
+  return fmaxf(0.f, fminf(fminf(2.f * r, 0.5f + 0.5f * r), 2.f));
+}
 template <typename T>
 __device__ __forceinline__ T mc_of(Native<T> &, T r) {
   const T a = T(2) * r, b = T(0.5) * (T(1) + r);
@@ -111,6 +116,7 @@ __device__ __forceinline__ T slope_limiter(M &m, int lim, T r, T eta) {
 // the limiter's value does not need it: num = +-0 gives r = +-0 exactly (sign
 // rule of IEEE division), and for minmod, MC, Superbee and Koren every
 // negative r gives phi = +0, so any negative stand-in does; "1st" ignores r.
+__device__ __forceinline__ float limiter_ratio(Quick &m, int, float num, float den) { return m.div(num, den); }
 template <typename T, class M>
 __device__ __forceinline__ T limiter_ratio(M &m, int lim, T num, T den) {
   if (lim == LIM_1ST) return T(0);
@@ -134,10 +140,10 @@ __device__ __forceinline__ void muscl_face(M &m, int lim, T wi, T wip, T dA, T d
     etaL = m.div(dB * dB + dA * dA, (T(1) * h) * (T(1) * h));
     etaR = m.div(dC * dC + dB * dB, (T(1) * h) * (T(1) * h));
   }
-  T r = limiter_ratio<T>(m, lim, dB, dA + E);
+  T r = limiter_ratio(m, lim, dB, dA + E);
   T phi = slope_limiter<T>(m, lim, r, etaL);
   left = wi + m.half(phi) * dA;
-  r = limiter_ratio<T>(m, lim, dB, dC + E);
+  r = limiter_ratio(m, lim, dB, dC + E);
   phi = slope_limiter<T>(m, lim, r, etaR);
   right = wip - m.half(phi) * dC;
 }
@@ -219,6 +225,15 @@ __device__ __forceinline__ T fast_speed(M &m, const T *w, T gamma, int norm) {
   return m.root(m.half(i0 + m.root(i1 * i1 + m.quad(a * a) * ((ca * ca) - (can * can)))));
 }
 
+// FP32 faces: the squares of the sound and Alfven speeds as they are, without
+// the roots that the FP64 path takes and squares again (fewer roundings)
+__device__ __forceinline__ float fast_speed_of(Quick &m, const float *w, float gamma, float b2) {
+  const float ir = m.div(1.f, w[0]);
+  const float c2 = b2 * ir, a2 = gamma * w[4] * ir, n2 = w[5] * w[5] * ir;
+  const float d = c2 - a2;
+  return m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (c2 - n2))));
+}
+
 // the same for norm 5 (x) and 6 (y), whose first two terms are the same values
 template <typename T, class M>
 __device__ __forceinline__ void fast_speeds(M &m, const T *w, T gamma, T *cf) {
@@ -248,6 +263,16 @@ __device__ __forceinline__ void side_scalars(M &m, const T *w, T gamma, T &cf, T
   e = m.div(w[4], w[0] * (gamma - T(1))) + m.half(w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) + m.half(m.div(b2, w[0]));
   e = e * w[0];
   pt = w[4] + m.half(b2);
+}
+
+// FP32 faces: the energy as p/(gamma - 1) + rho v^2/2 + B^2/2, without the
+// reference's detour over the energy per mass (fewer roundings)
+template <typename T>
+__device__ __forceinline__ void side_scalars(Quick &m, const float *w, float gamma, float &cf, float &pt, float &e) {
+  const float b2 = w[5] * w[5] + w[6] * w[6] + w[7] * w[7];
+  cf = fast_speed_of(m, w, gamma, b2);
+  e = m.div(w[4], gamma - 1.f) + 0.5f * (w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) + b2);
+  pt = w[4] + 0.5f * b2;
 }
 
 template <typename T, class M>

@@ -296,6 +296,24 @@ struct Soft {
   __device__ __forceinline__ bool nonzero(double a) { return (f64_bits(a) << 1) != 0; }
   __device__ __forceinline__ bool failed() const { return bad; }
 };
+// The FP32 face kernels': quotients and roots from MUFU without the
+// compiler's handling of subnormal operands (2 and 1 instructions; a quotient
+// is a * rcp(b), within 2 ulp, and quotients of one b share the reciprocal).
+struct Quick : Native<float> {
+  __device__ __forceinline__ float div(float a, float b) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return a * r;
+  }
+  __device__ __forceinline__ float root(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+  }
+  template <int B> __device__ __forceinline__ float by(float a) { return a * (1.0f / B); }
+};
+template <typename T> struct FaceArith { using type = Soft; };
+template <> struct FaceArith<float> { using type = Quick; };
 template <typename T> struct ArithOf { using type = Native<T>; };
 template <> struct ArithOf<double> { using type = Soft; };
 

@@ -58,12 +58,24 @@ __device__ __forceinline__ void dev_fail(DevError *e, int code, int blk, int i, 
 }
 
 // floor of the pressure recovered by the FP32 path (code units)
-constexpr double kPressureFloor = 1.0e-10;
+constexpr float kPressureFloor = 1.0e-10f;
 
-// meshblock.cpp:119-179 for one cell; the FP32 path recovers the pressure in
-// FP64 from the FP32 conserved state and floors it (positivity fix).
+// gamma as the primitive recovery of storage type S takes it
+template <typename S> struct GasGamma;
+template <> struct GasGamma<double> {
+  double g;
+  __device__ __forceinline__ GasGamma(const InstParams &p) : g(p.gamma) {}
+  __device__ __forceinline__ explicit GasGamma(double gamma) : g(gamma) {}
+};
+template <> struct GasGamma<float> {
+  float hi, lo;   // gamma - 1
+  __device__ __forceinline__ GasGamma(const InstParams &p) : hi(p.gm1_hi), lo(p.gm1_lo) {}
+};
+
+// meshblock.cpp:119-179 for one cell; the FP32 path recovers the pressure
+// from pairs of floats and floors it (positivity fix).
 template <typename S>
-__device__ __forceinline__ void cons2prim_cell(const S *u, S *w, double gamma);
+__device__ __forceinline__ void cons2prim_cell(const S *u, S *w, const GasGamma<S> &gam);
 
 template <class M>
 __device__ __forceinline__ void cons2prim_f64(M &m, const double *u, double *w, double g) {
@@ -71,82 +83,65 @@ __device__ __forceinline__ void cons2prim_f64(M &m, const double *u, double *w, 
   w[1] = m.div(u[1], u[0]);
   w[2] = m.div(u[2], u[0]);
   w[3] = m.div(u[3], u[0]);
-  double p = (g - 1) * (u[4] - 0.5 * w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]));
+  double p = (g - 1) * (u[4] - m.half(w[0]) * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]));
   w[5] = u[5];
   w[6] = u[6];
   w[7] = u[7];
-  w[4] = p - (g - 1) * (0.5 * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]));
+  w[4] = p - (g - 1) * m.half(u[5] * u[5] + u[6] * u[6] + u[7] * u[7]);
 }
 template <>
-__device__ __forceinline__ void cons2prim_cell<double>(const double *u, double *w, double g) {
-  evaluate<double>([&](auto &m) { cons2prim_f64(m, u, w, g); });
+__device__ __forceinline__ void cons2prim_cell<double>(const double *u, double *w, const GasGamma<double> &gam) {
+  evaluate<double>([&](auto &m) { cons2prim_f64(m, u, w, gam.g); });
 }
 
-// a^2 + b^2 + c^2 of FP32 values as an unevaluated sum hi + lo, exact to
-// about 2^-48 relative: each square split exactly by an FMA (Dekker's
-// product) and the partial sums by Knuth's TwoSum, with the error terms
-// summed in FP32.  The _rn intrinsics keep the compiler from fusing or
+// Pairs of floats.  The _rn intrinsics keep the compiler from fusing or
 // reordering the steps.
+// a + b = s + e exactly (Knuth's TwoSum)
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
+  s = __fadd_rn(a, b);
+  const float v = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v));
+}
+// a^2 + b^2 + c^2 as hi + lo, exact to about 2^-48 relative: each square split
+// exactly by an FMA (Dekker's product), the partial sums by TwoSum, with the
+// error terms summed in FP32
 __device__ __forceinline__ void sum_sq3(float a, float b, float c, float &hi, float &lo) {
   const float pa = __fmul_rn(a, a), pb = __fmul_rn(b, b), pc = __fmul_rn(c, c);
   const float ea = __fmaf_rn(a, a, -pa), eb = __fmaf_rn(b, b, -pb), ec = __fmaf_rn(c, c, -pc);
-  const float s1 = __fadd_rn(pa, pb), v1 = __fsub_rn(s1, pa);
-  const float t1 = __fadd_rn(__fsub_rn(pa, __fsub_rn(s1, v1)), __fsub_rn(pb, v1));
-  const float s2 = __fadd_rn(s1, pc), v2 = __fsub_rn(s2, s1);
-  const float t2 = __fadd_rn(__fsub_rn(s1, __fsub_rn(s2, v2)), __fsub_rn(pc, v2));
-  hi = s2;
+  float s1, t1, t2;
+  two_sum(pa, pb, s1, t1);
+  two_sum(s1, pc, hi, t2);
   lo = __fadd_rn(__fadd_rn(__fadd_rn(ea, eb), ec), __fadd_rn(t1, t2));
 }
 
-// FP32 path: the pressure recovered from the total energy in FP64 (the
-// cancellation E - |m|^2/2rho - |B|^2/2 is where FP32 loses digits).  The
-// sums of squares |m|^2 and |B|^2 and the quotient |m|^2/rho come from the
-// FP32 pipe as hi + lo pairs (sum_sq3, and the product with 1/rho = ir + rl),
-// accurate to ~2^-45, and are widened to FP64 only for E - (|m|^2/rho +
-// |B|^2)/2 and the factor gamma - 1.  On this GPU FP64 runs at 1/64 of the
-// FP32 rate: this takes a third of the FP64 operations of squaring, summing
-// and dividing in FP64.  AMR_PRESSURE_DF=1: |m|^2/rho with 1/rho refined by
-// one FP64 Newton step instead.
-// The velocities are the FP32 momenta times the FP32 reciprocal.  (A
-// component above ~1.8e19 overflows its FP32 square; such a state is out of
-// the FP32 path's range in any case.)  AMR_PRESSURE_DF=0 restores the FP64
-// squares and sums.
-#ifndef AMR_PRESSURE_DF
-#define AMR_PRESSURE_DF 2
-#endif
+// FP32 path: the pressure from the total energy, (gamma - 1) (E - (|m|^2/rho +
+// |B|^2)/2), whose cancellation is where FP32 loses digits, evaluated with
+// pairs of floats: the sums of squares (sum_sq3), |m|^2/rho with 1/rho = ir +
+// rl (rl from the FMA residual 1 - rho*ir), the sum of both halves and the
+// subtraction (TwoSum), and the product with gamma - 1 (a pair as well).
+// Every step is good to 2^-45 of the subtracted terms, which an evaluation
+// with FP64 sums does not improve on (the pairs it starts from carry that
+// error), and none is on the FP64 pipe, 12 instructions of which per cell kept
+// the FP32 path's dt kernel 76 % bound (16 clocks per warp each).  The
+// velocities are the FP32 momenta times the FP32 reciprocal.  (A component
+// above ~1.8e19 overflows its FP32 square; such a state is out of the FP32
+// path's range in any case.)
 template <>
-__device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, double g) {
+__device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, const GasGamma<float> &gam) {
   const float ir = 1.0f / u[0];
-#if AMR_PRESSURE_DF == 2
-  // |m|^2 / rho as hi + lo on the FP32 pipe too: 1/rho = ir + rl (rl from the
-  // FMA residual 1 - rho*ir, ~2^-45 relative), the product of the two pairs
-  // with Dekker's exact error term
   const float rl = __fmul_rn(__fmaf_rn(-u[0], ir, 1.0f), ir);
   float mh, ml, bh, bl;
   sum_sq3(u[1], u[2], u[3], mh, ml);
   sum_sq3(u[5], u[6], u[7], bh, bl);
   const float kh = __fmul_rn(mh, ir);
   const float kl = __fadd_rn(__fmaf_rn(mh, ir, -kh), __fadd_rn(__fmul_rn(mh, rl), __fmul_rn(ml, ir)));
-  double p = (g - 1) * (static_cast<double>(u[4]) -
-                        0.5 * ((static_cast<double>(kh) + static_cast<double>(kl)) +
-                               (static_cast<double>(bh) + static_cast<double>(bl))));
-#elif AMR_PRESSURE_DF
-  double ird = static_cast<double>(ir);
-  ird = __fma_rn(ird, __fma_rn(-static_cast<double>(u[0]), ird, 1.0), ird);
-  float mh, ml, bh, bl;
-  sum_sq3(u[1], u[2], u[3], mh, ml);
-  sum_sq3(u[5], u[6], u[7], bh, bl);
-  const double m2 = static_cast<double>(mh) + static_cast<double>(ml);
-  const double b2 = static_cast<double>(bh) + static_cast<double>(bl);
-  double p = (g - 1) * (static_cast<double>(u[4]) - 0.5 * (m2 * ird + b2));
-#else
-  double ird = static_cast<double>(ir);
-  ird = ird * (2.0 - static_cast<double>(u[0]) * ird);
-  const double mx = u[1], my = u[2], mz = u[3];
-  const double bx = u[5], by = u[6], bz = u[7];
-  double p = (g - 1) * (static_cast<double>(u[4]) - 0.5 * (mx * mx + my * my + mz * mz) * ird) -
-             (g - 1) * (0.5 * (bx * bx + by * by + bz * bz));
-#endif
+  float sh, sl, dh, dl;
+  two_sum(kh, bh, sh, sl);
+  sl = __fadd_rn(sl, __fadd_rn(kl, bl));
+  two_sum(u[4], __fmul_rn(-0.5f, sh), dh, dl);
+  dl = __fmaf_rn(-0.5f, sl, dl);
+  const float ph = __fmul_rn(gam.hi, dh);
+  float p = __fadd_rn(ph, __fadd_rn(__fmaf_rn(gam.hi, dh, -ph), __fmaf_rn(gam.hi, dl, __fmul_rn(gam.lo, dh))));
   // positivity fix of the FP32 path: the FP32 conserved state can put the
   // recovered pressure below zero where the FP64 path stays positive
   if (!(p > kPressureFloor)) p = kPressureFloor;
@@ -154,20 +149,24 @@ __device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, 
   w[1] = u[1] * ir;
   w[2] = u[2] * ir;
   w[3] = u[3] * ir;
-  w[4] = static_cast<float>(p);
+  w[4] = p;
   w[5] = u[5];
   w[6] = u[6];
   w[7] = u[7];
 }
 
 // FP32 fused stage: 320 threads per CTA (the 2 x 17 x 17 = 578 faces of a
-// block in two rounds; 256 threads take three, the last a quarter full),
-// compiled for 3 resident CTAs per SM (64 registers, ~120 B of spills to L1).
-// Timed on the 64-rotor FP32 batch (one GB300, 20 steps): 5.17 ms per step
-// against 5.52 ms at 256 threads / 4 CTAs, 5.57 ms at 320 / 2 CTAs (96
-// registers, no spills); the 512-blast batch 24.7 against 25.1 and 27.8 ms.
+// block in two rounds), compiled for 4 resident CTAs per SM (48 registers, 56 B
+// of spills).  It issues in 48 % of its cycles and waits on latency between its
+// phases, so residents pay.  One GB300, us per pass of 32 rotors (12 steps), 24
+// blasts (10 steps) and a 512^2 KH layer (8 steps), state transfers included:
+//   320 threads x 4 CTAs  19812  8127  2233      320 x 3  20696  8442  2404
+//   256 x 5               19776  8133  2286      192 x 6  19763  8172  2403
+//   160 x 6               19986  8275  2417      128 x 7  20600  8487  2527
+// The kernel itself on the 6272 blocks of the rotors: 460 us at first, 377 in
+// the face frame, 287 with Quick arithmetic and the pair recovery (3 CTAs).
 #ifndef AMR_STAGE_F32_MINB
-#define AMR_STAGE_F32_MINB 3
+#define AMR_STAGE_F32_MINB 4
 #endif
 #ifndef AMR_STAGE_F32_THREADS
 #define AMR_STAGE_F32_THREADS 320
@@ -324,7 +323,7 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
     S u[8], w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = sU[k * NN + c];
-    cons2prim_cell<S>(u, w, ip.gamma);
+    cons2prim_cell<S>(u, w, GasGamma<S>(ip));
 #pragma unroll
     for (int k = 0; k < 8; k++) sW[k * NN + c] = w[k];
     const int i = c % N, j = c / N;
@@ -358,7 +357,7 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
     const T h = static_cast<T>(yf ? task.dy : task.dx);
     const T bn = static_cast<T>(yf ? By[fpos] : Bx[fpos]);
     T fl[8];
-    typename ArithOf<T>::type m;
+    typename FaceArith<T>::type m;
     int rc = face_flux_of<RECON, FLUX, NN, T>(m, sW, cL, s, yf, lim, h, bn, gamma, fl);
     if (m.failed()) {
       T *out = (yf ? gg : ff) + fpos;
@@ -381,22 +380,29 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   __syncthreads();
 
   // 3. residual on [LO, HI]^2 (zero elsewhere) and the RK stage on every cell
-  const T dx = static_cast<T>(task.dx), dy = static_cast<T>(task.dy), dt = static_cast<T>(ip.dt);
+  const T dt = static_cast<T>(ip.dt);
+  // FP32: the rounded reciprocals once per block (a division per value has
+  // no less error); FP64: the reference's divisions
+  const T dx = static_cast<T>(sizeof(T) == 4 ? task.rcp_dx : task.dx);
+  const T dy = static_cast<T>(sizeof(T) == 4 ? task.rcp_dy : task.dy);
   S *out = static_cast<S *>(a.qout) + base;
-  for (int e = tid; e < 8 * NN; e += nthr) {
-    const int k = e / NN, c = e % NN;
+  for (int c = tid; c < NN; c += nthr) {   // all variables of a cell per thread: its index is decoded once
     const int i = c % N, j = c / N;
-    T res = T(0.);
-    if (i >= LO && i <= HI && j >= LO && j <= HI) {
-      const int cx = i - LO, r = j - LO;
-      evaluate<T>([&](auto &m) {
-        res = m.div(sFx[(k * NF + r) * NFX + cx + 1] - sFx[(k * NF + r) * NFX + cx], dx) +
-              m.div(sFy[(k * NFX + r + 1) * NF + cx] - sFy[(k * NFX + r) * NF + cx], dy);
-      });
+    const bool inside = i >= LO && i <= HI && j >= LO && j <= HI;
+    const T *fx = sFx + (inside ? (j - LO) * NFX + i - LO : 0), *fy = sFy + (inside ? (j - LO) * NF + i - LO : 0);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      T res = T(0.);
+      if (inside) {
+        const T gx = fx[k * NF * NFX + 1] - fx[k * NF * NFX], gy = fy[k * NFX * NF + NF] - fy[k * NFX * NF];
+        if (sizeof(T) == 4) res = gx * dx + gy * dy;
+        else evaluate<T>([&](auto &m) { res = m.div(gx, dx) + m.div(gy, dy); });
+      }
+      const int e = k * NN + c;
+      const T q = KEEPU ? sU[e] : Q[e];
+      if (a.step == 1) out[e] = q - dt * res;                         // Us = U - dt res
+      else out[e] = T(0.5) * (out[e] + q - dt * res);                 // U = (U + Us - dt res)/2
     }
-    const T q = KEEPU ? sU[e] : Q[e];
-    if (a.step == 1) out[e] = q - dt * res;                         // Us = U - dt res
-    else out[e] = T(0.5) * (out[e] + q - dt * res);                 // U = (U + Us - dt res)/2
   }
   // fused fill: snapshots of the next fill (ff, gg and B, whose writes by
   // this CTA precede the barrier after step 2)

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(512) k_prim(SplitArgs a) {
   S u[8], w[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) u[k] = Q[k * NN + c];
-  cons2prim_cell<S>(u, w, a.inst[task.inst].gamma);
+  cons2prim_cell<S>(u, w, GasGamma<S>(a.inst[task.inst]));
 #pragma unroll
   for (int k = 0; k < 8; k++) W[k * NN + c] = w[k];
   const int i = c % N, j = c / N;
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) k_prim_task(SplitArgs a) {
   const size_t base = static_cast<size_t>(task.slot) * 8 * NN;
   const S *Q = static_cast<const S *>(a.qin) + base;
   S *W = static_cast<S *>(a.W) + base;
-  const double gamma = a.inst[task.inst].gamma;
+  const GasGamma<S> gamma(a.inst[task.inst]);
   for (int c = threadIdx.x; c < NN; c += blockDim.x) {
     S u[8], w[8];
 #pragma unroll
@@ -112,7 +112,7 @@ __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
   const T bn = static_cast<T>(Bf[fpos]);
   S *out = static_cast<S *>(yf ? a.gg : a.ff) + base + fpos;
   T fl[8];
-  typename ArithOf<T>::type m;
+  typename FaceArith<T>::type m;
   int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, ip.limiter, h, bn, gamma, fl);
   if (m.failed()) {
     rc = face_flux_native<RECON, FLUX, NN, T>(W, cL, s, yf, ip.limiter, h, bn, gamma, out);

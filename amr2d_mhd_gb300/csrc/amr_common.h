@@ -84,7 +84,7 @@ struct InstParams {
 // (src_pos, src_pos + 1) of one source block; both positions even, so the
 // pair is one aligned 8-byte (float) or 16-byte (double) access.
 enum GhostOpType : uint8_t { GOP_COPY = 0, GOP_SNAP = 1, GOP_FINE = 2, GOP_SFINE = 3, GOP_NOP = 4, GOP_COPY2 = 5 };
-struct GhostOp {
+struct alignas(16) GhostOp {   // one 16-byte load
   int dst_slot;
   int src_slot;     // physical slot, or first snapshot row for SNAP / SFINE
   int16_t dst_pos;  // j * N + i within the block plane

@@ -60,18 +60,18 @@ struct CtArgs {
 };
 
 // prologue and epilogue of a per-block kernel of the step with fused fills
-template <int N>
+template <int N, typename S>
 __device__ __forceinline__ void fuse_apply(const FillFuse &f, const LeafTask &t) {
   if (f.apply.nseg) {
-    fill_apply_task<N, double>(f, t, threadIdx.x, blockDim.x, nullptr);
+    fill_apply_task<N, S>(f, t, block_tid(), blockDim.x);
     __syncthreads();
   }
 }
-template <int N>
+template <int N, typename S>
 __device__ __forceinline__ void fuse_save(const FillFuse &f, const LeafTask &t) {
   if (f.save.nseg) {
     __syncthreads();
-    fill_save_task<N>(f, t, threadIdx.x, blockDim.x);
+    fill_save_task<N, S>(f, t, block_tid(), blockDim.x);
   }
 }
 
@@ -90,14 +90,14 @@ __device__ __forceinline__ void ct_emf_upwind(const CtArgs &a, const LeafTask &t
   const S *ff = static_cast<const S *>(a.ff) + static_cast<size_t>(t.slot) * 8 * NN;
   const S *gg = static_cast<const S *>(a.gg) + static_cast<size_t>(t.slot) * 8 * NN;
   double *E = a.EMF + static_cast<size_t>(t.slot) * NN;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = block_tid(); c < NN; c += blockDim.x) {
     const S q0 = q[c], q1 = q[NN + c], q2 = q[2 * NN + c], q3 = q[3 * NN + c];
     const S q4 = q[4 * NN + c], q5 = q[5 * NN + c], q6 = q[6 * NN + c], q7 = q[7 * NN + c];
     sp[c] = (g - S(1)) * (q4 - S(0.5) * ((q1 * q1 + q2 * q2 + q3 * q3) / q0 + (q5 * q5 + q6 * q6 + q7 * q7)));
     sC[c] = sqrt((g * sp[c] + (q5 * q5 + q6 * q6 + q7 * q7)) / q0);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = block_tid(); c < NN; c += blockDim.x) {
     const int i = c % N, j = c / N;
     if (i < 1 || j < 1) continue;
     const int w = c - 1, s = c - N, sw = c - N - 1;  // (i-1,j), (i,j-1), (i-1,j-1)
@@ -128,16 +128,16 @@ __device__ __forceinline__ void ct_emf_upwind(const CtArgs &a, const LeafTask &t
 template <int NG, typename S>
 __device__ __forceinline__ void ct_emf_block(const CtArgs &a, const FillFuse &f, const LeafTask &t, S *sp, S *sC) {
   constexpr int N = Geo<NG>::N, NN = N * N;
-  fuse_apply<N>(f, t);
+  fuse_apply<N, S>(f, t);
   if (a.inst[t.inst].ct_type == 2) {
     ct_emf_upwind<NG, S>(a, t, sp, sC);
-    fuse_save<N>(f, t);
+    fuse_save<N, S>(f, t);
     return;
   }
   const S *ff = static_cast<const S *>(a.ff) + static_cast<size_t>(t.slot) * 8 * NN;
   const S *gg = static_cast<const S *>(a.gg) + static_cast<size_t>(t.slot) * 8 * NN;
   double *E = a.EMF + static_cast<size_t>(t.slot) * NN;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = block_tid(); c < NN; c += blockDim.x) {
     const int i = c % N, j = c / N;
     if (i < 1 || j < 1) continue;
     // in the storage type of the fluxes: FP64 on the FP64 path (the
@@ -148,19 +148,19 @@ __device__ __forceinline__ void ct_emf_block(const CtArgs &a, const FillFuse &f,
     const S f6a = ff[6 * NN + (j - 1) * N + i], f6b = ff[6 * NN + c];
     E[c] = static_cast<double>(S(0.25) * ((g5a + g5b) - (f6a + f6b)));
   }
-  fuse_save<N>(f, t);
+  fuse_save<N, S>(f, t);
 }
 
 // CT2D.cpp:78-92 face update with the RK2 combine
-template <int NG>
+template <int NG, typename S>
 __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f, const LeafTask &t) {
   constexpr int N = Geo<NG>::N, NN = N * N;
-  fuse_apply<N>(f, t);
+  fuse_apply<N, S>(f, t);
   const double dt = a.inst[t.inst].dt;
   const double *E = a.EMF + static_cast<size_t>(t.slot) * NN;
   const double *B0 = a.Bsrc + static_cast<size_t>(t.slot) * 2 * NN;
   double *B1 = a.Bnew + static_cast<size_t>(t.slot) * 2 * NN;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = block_tid(); c < NN; c += blockDim.x) {
     const int i = c % N, j = c / N;
     const int ip = i < N - 1 ? i + 1 : i, jp = j < N - 1 ? j + 1 : j;
     double res = t.rcp_dy * (E[jp * N + i] - E[c]);
@@ -170,7 +170,7 @@ __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f
     if (a.step == 1) B1[NN + c] = B0[NN + c] - dt * res;
     else B1[NN + c] = 0.5 * (B0[NN + c] + B1[NN + c] - dt * res);
   }
-  fuse_save<N>(f, t);
+  fuse_save<N, S>(f, t);
 }
 
 // CT2D.cpp:95-123 cell B := face average, with the energy correction, on
@@ -178,10 +178,10 @@ __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f
 template <int NG, typename S>
 __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f, const LeafTask &t) {
   constexpr int N = Geo<NG>::N, NN = N * N;
-  fuse_apply<N>(f, t);
+  fuse_apply<N, S>(f, t);
   const double *B = a.Bnew + static_cast<size_t>(t.slot) * 2 * NN;
   S *q = static_cast<S *>(a.q) + static_cast<size_t>(t.slot) * 8 * NN;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = block_tid(); c < NN; c += blockDim.x) {
     const int i = c % N, j = c / N;
     const int ip = i < N - 1 ? i + 1 : i, ii = ip - 1;
     const int jp = j < N - 1 ? j + 1 : j, jj = jp - 1;
@@ -194,7 +194,7 @@ __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f
     q[5 * NN + c] = bx;
     q[6 * NN + c] = by;
   }
-  fuse_save<N>(f, t);
+  fuse_save<N, S>(f, t);
 }
 
 template <int NG, typename S>
@@ -205,10 +205,10 @@ __global__ void k_ct_emf(CtArgs a) {
   ct_emf_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x], sp, sC);
 }
 
-template <int NG>
+template <int NG, typename S>
 __global__ void k_ct_face(CtArgs a) {
   pdl_wait();
-  ct_face_block<NG>(a, a.fuse, a.tasks[blockIdx.x]);
+  ct_face_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x]);
 }
 
 template <int NG, typename S>
@@ -255,7 +255,11 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, DevError *err) {
 // face field) are fused: gathered by the phase that consumes them, their
 // snapshots saved by the phase before.  The EMF phase also gathers the fill
 // of the fluxes and face field that precedes CT2D (main.cpp:161-163), and
-// the cell phase saves the snapshots of the cell fill that follows it.
+// the cell phase saves the snapshots of the cell fill that follows it.  Bound
+// by the latency of the gathers: with groups of variables per thread and wide
+// CTAs for few leaves (launch_ct_coop) 6272 FP32 leaves take 240 us (268
+// before), 196 take 23 (33), 196 FP64 leaves 26 (37).  Registers are held to 40
+// (FP32) and 64 for the resident warps.
 template <int NG, typename S, int THREADS>
 __global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1536 : 1024) / THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
                                                      unsigned *bar) {
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1536 : 1024) / THRE
     __syncthreads();  // the upwind form's shared scratch is reused by the next task
   }
   if (!grid_barrier(bar, a.err)) return;
-  for (int ti = blockIdx.x; ti < a.ntasks; ti += gridDim.x) ct_face_block<NG>(a, f_face, a.tasks[ti]);
+  for (int ti = blockIdx.x; ti < a.ntasks; ti += gridDim.x) ct_face_block<NG, S>(a, f_face, a.tasks[ti]);
   if (!grid_barrier(bar, a.err)) return;
   for (int ti = blockIdx.x; ti < a.ntasks; ti += gridDim.x) ct_cell_block<NG, S>(a, f_cell, a.tasks[ti]);
 }
@@ -361,7 +365,7 @@ __global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a
   __shared__ double red[2][8];
   __shared__ S sW[8 * NN];
   const LeafTask t = a.tasks[blockIdx.x];
-  fuse_apply<N>(a.fuse, t);
+  fuse_apply<N, S>(a.fuse, t);
   const S *U = static_cast<const S *>(a.U) + static_cast<size_t>(t.slot) * 8 * NN;
   for (int c = threadIdx.x; c < NN; c += blockDim.x) {
     S u[8], w[8];

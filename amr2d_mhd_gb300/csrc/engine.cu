@@ -566,7 +566,7 @@ FillPass Engine::fill_pass(std::initializer_list<std::pair<FillKind, int>> what,
     g.nv = field_nv(w.second);
     g.kind = w.first;
     g.f32 = field_f32(w.second) ? 1 : 0;
-    p.rows += g.nv;
+    p.groups += row_groups(g.nv, g.f32);
   }
   p.nseg = q;
   p.tile_seg = tile_seg;

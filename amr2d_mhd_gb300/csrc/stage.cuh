@@ -277,7 +277,7 @@ template <> struct StageKeepU<float> { static constexpr bool value = AMR_STAGE_F
 // caller) in phase `phase`.  Returns false (after recording DERR_TIMEOUT and
 // letting the copy land) when the bounded wait gave up; the decision is the
 // same in every thread of the CTA.
-template <int NG, int RECON, int FLUX, typename S>
+template <int NG, int RECON, int FLUX, typename S, bool PRE>
 __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t *bar, uint32_t phase) {
   using G = Geo<NG>;
   using T = S;
@@ -297,13 +297,17 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   S *gg = static_cast<S *>(a.gg) + base;
   const double *Bx = a.B + static_cast<size_t>(task.slot) * 2 * NN;
   const double *By = Bx + NN;
-  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int tid = block_tid(), nthr = blockDim.x;
 
   // 0. the block's conserved state (8 planes, contiguous) into shared memory by TMA
   static_assert((8 * NN * sizeof(S)) % 16 == 0, "bulk copies move multiples of 16 bytes");
   if (tid == 0) bulk_stage_issue(sU, Q, static_cast<uint32_t>(8 * NN * sizeof(S)), bar);
-  // fused fill: each thread's first gather is loaded while the copy is in flight
-  const FillPre pre = fill_prefetch<N>(a.fuse, task, tid);
+  // fused fill: each thread's first gathers are loaded while the copy is in
+  // flight (not in the loop of k_stage_dyn, where the values held over the wait
+  // spill)
+  FillPre<S> pre;
+  pre.on = false;
+  if (PRE) fill_prefetch<N, S>(a.fuse, task, tid, pre);
   const bool late = !bulk_stage_wait(bar, phase);
   if (__syncthreads_or(late)) {
     if (tid == 0) dev_fail(a.err, DERR_TIMEOUT, task.slot, 0, 0, 0.0);
@@ -406,7 +410,7 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   }
   // fused fill: snapshots of the next fill (ff, gg and B, whose writes by
   // this CTA precede the barrier after step 2)
-  if (a.fuse.save.nseg) fill_save_task<N>(a.fuse, task, tid, nthr);
+  if (a.fuse.save.nseg) fill_save_task<N, S>(a.fuse, task, tid, nthr);
   return true;
 }
 
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::val
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   stage_bar_init(&bar);
-  stage_block<NG, RECON, FLUX, S>(a, blockIdx.x, &bar, 0);
+  stage_block<NG, RECON, FLUX, S, true>(a, blockIdx.x, &bar, 0);
 }
 
 // persistent: a grid of the CTAs the SMs hold at once sweeps the leaf list of
@@ -442,7 +446,7 @@ __global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::val
     __syncthreads();
     const int ti = next;
     if (ti >= a.ntasks) break;
-    if (!stage_block<NG, RECON, FLUX, S>(a, ti, &bar, it & 1u)) break;
+    if (!stage_block<NG, RECON, FLUX, S, false>(a, ti, &bar, it & 1u)) break;
     __syncthreads();  // shared memory free for the next block's copy
   }
   if (threadIdx.x == 0) {

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_prim_task(SplitArgs a) {
   using G = Geo<NG>;
   constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI;
   const LeafTask task = a.tasks[blockIdx.x];
-  fill_apply_task<N, double>(a.fuse, task, threadIdx.x, blockDim.x, nullptr);
+  fill_apply_task<N, S>(a.fuse, task, threadIdx.x, blockDim.x);
   __syncthreads();
   const size_t base = static_cast<size_t>(task.slot) * 8 * NN;
   const S *Q = static_cast<const S *>(a.qin) + base;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(512) k_resid(SplitArgs a) {
   constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI;
   const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   // fused fill: the flux fill's snapshots (this kernel writes only qout)
-  if (a.fuse.save.nseg) fill_save_all<N>(a.fuse, e, static_cast<size_t>(gridDim.x) * blockDim.x);
+  if (a.fuse.save.nseg) fill_save_all<N, S>(a.fuse, e, static_cast<size_t>(gridDim.x) * blockDim.x);
   if (e >= static_cast<size_t>(a.ntasks) * 8 * NN) return;
   const int t = static_cast<int>(e / (8 * NN)), r = static_cast<int>(e % (8 * NN));
   const int c = r % NN;

@@ -51,6 +51,20 @@ cudaError_t launch_faces(const Method &m, const SplitArgs &a, cudaStream_t s) {
 }
 
 namespace {
+// Up to two leaves per SM: the kernels with one CTA per leaf take 512 threads
+// instead of 256, as their time is that of one leaf's rounds of cells (196
+// leaves: k_prim_task 13.6 -> 12.6 us, FP32 k_dt_cell 10.3 -> 9.2; 40-leaf
+// Brio-Wu program 6293 -> 6165 us with both)
+bool wide_cta(int ntasks) {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 0;
+  }
+  return ntasks <= 2 * sms;
+}
 int cell_threads(const Method &m) { return m.cell_block == 128 || m.cell_block == 512 ? m.cell_block : 256; }
 }  // namespace
 
@@ -59,10 +73,11 @@ cudaError_t launch_prim(const Method &m, const SplitArgs &a, cudaStream_t s) {
   const size_t n = static_cast<size_t>(a.ntasks) * nn;
   if (n == 0) return cudaSuccess;
   if (a.fuse.apply.nseg) {  // fused fill: one CTA per leaf
-    if (m.ng == 2 && !m.f32) return launch_k(m.pdl, k_prim_task<2, double>, a.ntasks, 256, 0, s, a);
-    if (m.ng == 2) return launch_k(m.pdl, k_prim_task<2, float>, a.ntasks, 256, 0, s, a);
-    if (!m.f32) return launch_k(m.pdl, k_prim_task<4, double>, a.ntasks, 256, 0, s, a);
-    return launch_k(m.pdl, k_prim_task<4, float>, a.ntasks, 256, 0, s, a);
+    const int w = wide_cta(a.ntasks) ? 512 : 256;
+    if (m.ng == 2 && !m.f32) return launch_k(m.pdl, k_prim_task<2, double>, a.ntasks, w, 0, s, a);
+    if (m.ng == 2) return launch_k(m.pdl, k_prim_task<2, float>, a.ntasks, w, 0, s, a);
+    if (!m.f32) return launch_k(m.pdl, k_prim_task<4, double>, a.ntasks, w, 0, s, a);
+    return launch_k(m.pdl, k_prim_task<4, float>, a.ntasks, w, 0, s, a);
   }
   const int b = cell_threads(m);
   const unsigned g = static_cast<unsigned>((n + b - 1) / b);
@@ -198,6 +213,7 @@ cudaError_t launch_ct_cell(const Method &m, const CtArgs &a, int n, cudaStream_t
 
 cudaError_t launch_dt_cell(const Method &m, const DtArgs &a, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
+  if (wide_cta(n)) return AMR_DISPATCH_NG_S_PDL(m, k_dt_cell_wide, n, 512, 0, s, a);
   return AMR_DISPATCH_NG_S_PDL(m, k_dt_cell, n, 256, 0, s, a);
 }
 

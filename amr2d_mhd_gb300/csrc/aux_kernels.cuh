@@ -352,12 +352,10 @@ struct DtArgs {
   FillFuse fuse;    // fused fills: the fill of U after the step, gathered first
 };
 
-// resident CTAs of k_dt_cell: the FP32 form has to hide its loads (32 registers)
-template <typename S> struct DtMinBlocks { static constexpr int value = 5; };
-template <> struct DtMinBlocks<float> { static constexpr int value = 8; };
-template <int NG, typename S>
-__global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a) {
-  pdl_wait();
+// THREADS: 256, one thread per interior cell, or 512 for few leaves: then the
+// second 256 take the criterion while the first take the wave speeds
+template <int NG, typename S, int THREADS>
+__device__ __forceinline__ void dt_cell(const DtArgs &a) {
   using G = Geo<NG>;
   using T = S;
   constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI;
@@ -367,7 +365,7 @@ __global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a
   const LeafTask t = a.tasks[blockIdx.x];
   fuse_apply<N, S>(a.fuse, t);
   const S *U = static_cast<const S *>(a.U) + static_cast<size_t>(t.slot) * 8 * NN;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
+  for (int c = threadIdx.x; c < NN; c += THREADS) {
     S u[8], w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) u[k] = U[k * NN + c];
@@ -379,42 +377,50 @@ __global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a
       dev_fail(a.err, DERR_PRESSURE, t.slot, i, j, static_cast<double>(w[4]));
     bool bad = false;
 #pragma unroll
-    for (int k = 0; k < 8; k++) bad |= isnan(w[k]);
+    for (int k = 0; k < 8; k++) bad |= bits_nan(w[k]);
     if (bad) dev_fail(a.err, DERR_NAN, t.slot, i, j, 0.0);
   }
   __syncthreads();
-  const T g = static_cast<T>(a.inst[t.inst].gamma);
-  const int i = NG + threadIdx.x % NI, j = NG + threadIdx.x / NI, c = j * N + i;
+  const int cell = threadIdx.x % 256;
+  const int c = (NG + cell / NI) * N + NG + cell % NI;
   const S *W = sW;
-  T w[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) w[k] = W[k * NN + c];
+  const int lane = threadIdx.x & 31, wid = cell >> 5;
   // wavespeeds (misc.cpp:71-79) for norm 5 and 6; lambda1 takes |rho|
   // (main.cpp:222), lambda2 |u|.  The maxima in the storage type, widened to
   // FP64 once per warp: the widening is exact and monotonic, so this equals
   // the maximum of the widened values (and keeps FP32 maxima off the FP64 pipe).
-  T lamT = T(0.), grT = T(0.);
-  evaluate<T>([&](auto &m) {
-    T cf[2];
-    fast_speeds<T>(m, w, g, cf);
-    lamT = smax(fabs(w[0]) + cf[0], fabs(w[1]) + cf[1]);
-    grT = T(0.);
-    if (!a.want_grad) return;
+  if (threadIdx.x < 256) {
+    const T g = static_cast<T>(a.inst[t.inst].gamma);
+    T w[8];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int v = q == 0 ? 4 : (q == 1 ? 0 : q + 3);   // p, rho, Bx, By
-      const S *x = W + v * NN + c;
-      const T c0 = x[0];
-      const T dm = m.most(static_cast<T>(EPS), fabs(c0));
-      const T d1 = m.most(fabs(x[1] - c0), fabs(x[-1] - c0));
-      const T d2 = m.most(fabs(x[N] - c0), fabs(x[-N] - c0));
-      grT = m.most(grT, m.div(m.most(d1, d2), dm));
-    }
-  });
-  const double lam = static_cast<double>(warp_max_t(lamT));
-  const double gr = static_cast<double>(warp_max_t(grT));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { red[0][wid] = lam; red[1][wid] = gr; }
+    for (int k = 0; k < 8; k++) w[k] = W[k * NN + c];
+    T lamT = T(0.);
+    evaluate<T>([&](auto &m) {
+      T cf[2];
+      fast_speeds<T>(m, w, g, cf);
+      lamT = smax(fabs(w[0]) + cf[0], fabs(w[1]) + cf[1]);
+    });
+    const double lam = static_cast<double>(warp_max_t(lamT));
+    if (lane == 0) red[0][wid] = lam;
+  }
+  if (THREADS == 256 || threadIdx.x >= 256) {
+    T grT = T(0.);
+    if (a.want_grad) evaluate<T>([&](auto &m) {
+      grT = T(0.);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int v = q == 0 ? 4 : (q == 1 ? 0 : q + 3);   // p, rho, Bx, By
+        const S *x = W + v * NN + c;
+        const T c0 = x[0];
+        const T dm = m.most(static_cast<T>(EPS), fabs(c0));
+        const T d1 = m.most(fabs(x[1] - c0), fabs(x[-1] - c0));
+        const T d2 = m.most(fabs(x[N] - c0), fabs(x[-N] - c0));
+        grT = m.most(grT, m.div(m.most(d1, d2), dm));
+      }
+    });
+    const double gr = static_cast<double>(warp_max_t(grT));
+    if (lane == 0) red[1][wid] = gr;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     double mm = red[0][0], gg = red[1][0];
@@ -425,6 +431,20 @@ __global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a
     a.lambda[blockIdx.x] = mm;
     a.grad[blockIdx.x] = gg;
   }
+}
+
+// resident CTAs of k_dt_cell: the FP32 form has to hide its loads (32 registers)
+template <typename S> struct DtMinBlocks { static constexpr int value = 5; };
+template <> struct DtMinBlocks<float> { static constexpr int value = 8; };
+template <int NG, typename S>
+__global__ void __launch_bounds__(256, DtMinBlocks<S>::value) k_dt_cell(DtArgs a) {
+  pdl_wait();
+  dt_cell<NG, S, 256>(a);
+}
+template <int NG, typename S>
+__global__ void __launch_bounds__(512) k_dt_cell_wide(DtArgs a) {
+  pdl_wait();
+  dt_cell<NG, S, 512>(a);
 }
 
 // ------------------------------------------------- initial condition (amr_init)

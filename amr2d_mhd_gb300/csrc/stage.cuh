@@ -422,9 +422,11 @@ __device__ __forceinline__ void stage_bar_init(uint64_t *bar) {
   __syncthreads();
 }
 
-// one CTA per leaf block
-template <int NG, int RECON, int FLUX, typename S>
-__global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::value) k_stage(StageArgs a) {
+// One CTA per leaf block.  THREADS: StageThreads, or kStageWide for FP32 and
+// few blocks, whose 640 threads take the 578 faces in one round.
+constexpr int kStageWide = 640;
+template <int NG, int RECON, int FLUX, typename S, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinBlocks<S>::value) k_stage(StageArgs a) {
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   stage_bar_init(&bar);

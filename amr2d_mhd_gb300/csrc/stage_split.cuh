@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(512) k_prim(SplitArgs a) {
 // the same with the fill of qin (and B) fused in: one CTA per leaf gathers
 // its block's ghost cells, then converts the block
 template <int NG, typename S>
-__global__ void __launch_bounds__(256) k_prim_task(SplitArgs a) {
+__global__ void __launch_bounds__(512) k_prim_task(SplitArgs a) {
   pdl_wait();
   using G = Geo<NG>;
   constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI;

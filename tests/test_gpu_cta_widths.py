@@ -20,7 +20,7 @@ def uniform(gpu, roots, precision):
 @pytest.mark.parametrize("roots", [4, 16, 18, 20, 26, 36])
 def test_fp64_meshes_match_the_oracle(gpu, roots):
     c = uniform(gpu, roots, "fp64")
-    sim, orc = gpu.Simulation(c).init(), P.Oracle(**oracle_kw(c)).init()
+    sim, orc = gpu.Simulation(c).init(), P.Oracle(**oracle_kw(c), lenx=c.lenx, leny=c.leny).init()
     for _ in range(4):   # the first steps have dt = 0
         sim.step()
         orc.step()

@@ -117,6 +117,13 @@ __device__ __forceinline__ T slope_limiter(M &m, int lim, T r, T eta) {
 // rule of IEEE division), and for minmod, MC, Superbee and Koren every
 // negative r gives phi = +0, so any negative stand-in does; "1st" ignores r.
 __device__ __forceinline__ float limiter_ratio(Quick &m, int, float num, float den) { return m.div(num, den); }
+// FP64 faces: always the division, so that those of a face's variables overlap
+// (a branch around each puts them one after the other: KH 256 blocks 90 against
+// 79 us, 196-block rotor, with uniform regions a branch could skip, 109 against
+// 95, one warp alone 26.7 against 21.7)
+__device__ __forceinline__ double limiter_ratio(Soft &m, int lim, double num, double den) {
+  return lim == LIM_1ST ? 0.0 : m.div(num, den);
+}
 template <typename T, class M>
 __device__ __forceinline__ T limiter_ratio(M &m, int lim, T num, T den) {
   if (lim == LIM_1ST) return T(0);

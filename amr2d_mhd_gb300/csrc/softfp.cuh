@@ -11,9 +11,9 @@
 // GB300, 12 warps per SM: 26 clocks per SM and warp for an addition and a
 // division (115 with the compiler's), 25 for an addition and a square root
 // (115).  The face kernel with the Soft arithmetic, 196-block rotor (MC +
-// HLLD): 257 -> 100 us and 3.57 -> 1.43 M FP64-pipe instructions; 256-block KH
-// layer (MC + RUSA): 207 -> 92 us; 256-block Orszag-Tang (WENO5 + HLLD): 790
-// -> 300 us.
+// HLLD): 257 -> 90 us; 256-block KH layer (MC + RUSA): 207 -> 79 us and 2.87 ->
+// 1.12 M FP64-pipe instructions; 256-block Orszag-Tang (WENO5 + HLLD): 790 ->
+// 280 us.
 //
 // Method (long division with a large radix, two digits; e.g. Ercegovac &
 // Lang, Digital Arithmetic, ch. 5 and 7): a 23-bit reciprocal from MUFU,

@@ -219,6 +219,20 @@ __device__ __forceinline__ int face_plane(int k, bool yf) {
   return yf ? r : k;
 }
 
+// The left and right MUSCL states of a face, variables 0-4, 6, 7 of the face
+// frame.  LIM: a limiter known at compile time, which lets the variables'
+// chains overlap, or -1 for the one in `lim`.
+template <int LIM, int NN, typename T, class M>
+__device__ __forceinline__ void muscl_states(M &m, const T *W, int cL, int s, bool yf, int lim, T h, T *wl, T *wr) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    if (k == 5) continue;
+    const T *w = W + face_plane(k, yf) * NN + cL;
+    const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
+    muscl_face<T>(m, LIM >= 0 ? LIM : lim, w0, w1, w0 - wm, w1 - w0, w2 - w1, h, wl[k], wr[k]);
+  }
+}
+
 // MUSCL2D.cpp:24-116 for one face: W is plane 0 of the block's primitive
 // state (planes NN apart), cL the cell on its left (below it), s the cell
 // stride along its normal, yf whether that is y; bn the face's own normal
@@ -229,14 +243,15 @@ template <int RECON, int FLUX, int NN, typename T, class M>
 __device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma,
                                             T *fl) {
   T wl[8], wr[8];
+  if (RECON == REC_MUSCL) {
+    if (lim == LIM_MC) muscl_states<LIM_MC, NN, T>(m, W, cL, s, yf, lim, h, wl, wr);
+    else muscl_states<-1, NN, T>(m, W, cL, s, yf, lim, h, wl, wr);
+  }
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    if (k == 5) continue;
+    if (RECON == REC_MUSCL || k == 5) continue;
     const T *w = W + face_plane(k, yf) * NN + cL;
-    if (RECON == REC_MUSCL) {
-      const T wm = w[-s], w0 = w[0], w1 = w[s], w2 = w[2 * s];
-      muscl_face<T>(m, lim, w0, w1, w0 - wm, w1 - w0, w2 - w1, h, wl[k], wr[k]);
-    } else if (RECON == REC_WENO3) {
+    if (RECON == REC_WENO3) {
       T dummy;
       weno3_cell<T>(m, w[-s], w[0], w[s], wl[k], dummy);
       weno3_cell<T>(m, w[0], w[s], w[2 * s], dummy, wr[k]);

@@ -4,10 +4,9 @@
 // Some hosts cannot call cudaMalloc at the point where they need the time step:
 // code running inside a captured CUDA graph, allocator-free real-time loops,
 // or frameworks that own every device allocation and forbid others.  This
-// entry point takes the caller's device arrays and keeps its only scratch --
-// one partial result per block -- in a fixed array in this file's device
-// globals, so it allocates nothing.  Every GPU that loads the library holds
-// that array (kCflStaticMaxBlocks doubles, 512 KiB) until the process exits.
+// entry point takes the caller's device arrays and keeps its only scratch, the
+// running minimum and two counts, in this file's device globals, so it
+// allocates nothing.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -20,108 +19,102 @@ namespace amr {
 
 constexpr int kCflStaticMaxBlocks = 1 << 16;
 
-// per-block min(dx,dy)/lambda_b of the last call; shared by every call
-static __device__ __align__(256) double g_cfl_scratch[kCflStaticMaxBlocks];
+// The minimum over the blocks so far, as a key whose unsigned order is the
+// order of the values, the number of NaN blocks and of finished CTAs; shared
+// by every call.  The last CTA of a launch writes the result and puts the
+// start values back, so a call needs no other launch.
+constexpr unsigned long long kCflKeyMax = ~0ull;
+static __device__ unsigned long long g_cfl_key = kCflKeyMax;
+static __device__ unsigned g_cfl_nans = 0, g_cfl_done = 0;
 
-// Bound by the FP64 pipe (83 % busy): about 80 FP64 instructions per cell
-// with the divisions and square roots on the integer pipe (softfp.cuh), 240
-// with the compiler's; 20011 blocks take 0.77 ms, 2.25 ms before, where the
-// bytes would take 0.05 ms.
-// main.cpp:211-228 for one block of the dense array: lambda1 takes |rho| +
-// c_f,x (W[..][0], main.cpp:222) and lambda2 |u| + c_f,y (:224) over the
-// interior cells
-template <int NG>
-__global__ void __launch_bounds__(256) k_cfl_static_blocks(const double *U, const double *dxdy, double gamma,
-                                                           double *scratch) {
-  constexpr int N = Geo<NG>::N, NN = N * N, HI = Geo<NG>::HI;
-  __shared__ double red[8];
-  const double *u0 = U + static_cast<size_t>(blockIdx.x) * 8 * NN;
-  double m = 0.;
-  for (int c = threadIdx.x; c < NN; c += blockDim.x) {
-    const int i = c % N, j = c / N;
-    if (i < NG || i > HI || j < NG || j > HI) continue;
-    double u[8], w[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) u[k] = u0[k * NN + c];
-    cons2prim_cell<double>(u, w, GasGamma<double>(gamma));
-    double v1 = 0, v2 = 0;
-    evaluate<double>([&](auto &ar) {
-      double cf[2];
-      fast_speeds<double>(ar, w, gamma, cf);
-      v1 = fabs(w[0]) + cf[0];
-      v2 = fabs(w[1]) + cf[1];
-    });
-    // a NaN speed (e.g. a negative pressure) poisons the block's value
-    m = (isnan(v1) || isnan(v2)) ? NAN : smax(smax(m, v1), v2);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_xor_sync(0xffffffffu, m, o);
-    m = (isnan(v) || isnan(m)) ? NAN : (m < v ? v : m);
-  }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double mm = red[0];
-    for (int q = 1; q < static_cast<int>(blockDim.x >> 5); q++)
-      mm = (isnan(red[q]) || isnan(mm)) ? NAN : (mm < red[q] ? red[q] : mm);
-    scratch[blockIdx.x] = smin(dxdy[2 * blockIdx.x], dxdy[2 * blockIdx.x + 1]) / mm;
-  }
+__device__ __forceinline__ unsigned long long cfl_key(double v) {
+  const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
+  return u >> 63 ? ~u : u | (1ull << 63);
+}
+__device__ __forceinline__ double cfl_unkey(unsigned long long k) {
+  return __longlong_as_double(static_cast<long long>(k >> 63 ? k & ~(1ull << 63) : ~k));
 }
 
-// lambda = min(1e6, min over blocks) (main.cpp:209,228); a NaN block value
-// makes the result NaN, which the caller's invalid-dt check catches
-__global__ void k_cfl_static_min(const double *scratch, int n, double *out) {
-  __shared__ double red[32];
-  double m = 1.E6;
-  bool nan = false;
-  for (int b = threadIdx.x; b < n; b += blockDim.x) {
-    const double v = scratch[b];
-    nan |= isnan(v);
-    m = v < m ? v : m;
-  }
-  nan = __syncthreads_or(nan);
+// Bound by the FP64 pipe: about 35 FP64 instructions per cell, the divisions
+// and square roots on the integer pipe (softfp.cuh), and the maximum, where a
+// NaN counts as the largest, on the bit patterns.  One thread per interior
+// cell; the minimum over the blocks by an atomic of each CTA, taken over by
+// the last one.  20011 blocks: 0.37 ms (0.72 with a
+// loop over all cells of a block and a second launch for the minimum, 2.25 at
+// first), 64 blocks 9 us (18, 29).
+//
+// main.cpp:211-228 for one block of the dense array: lambda1 takes |rho| +
+// c_f,x (W[..][0], main.cpp:222) and lambda2 |u| + c_f,y (:224) over the
+// interior cells; lambda = min(1e6, min over blocks) (main.cpp:209,228); a
+// NaN block value makes the result NaN, which the caller's invalid-dt check
+// catches
+template <int NG>
+__global__ void __launch_bounds__(256) k_cfl_static(const double *U, const double *dxdy, double gamma, double *out) {
+  constexpr int N = Geo<NG>::N, NN = N * N;
+  static_assert(NI * NI == 256, "one thread per interior cell");
+  __shared__ unsigned long long red[8];
+  const double *u0 = U + static_cast<size_t>(blockIdx.x) * 8 * NN;
+  const int c = (NG + threadIdx.x / NI) * N + NG + threadIdx.x % NI;
+  double u[8], w[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) u[k] = u0[k * NN + c];
+  cons2prim_cell<double>(u, w, GasGamma<double>(gamma));
+  double v1 = 0, v2 = 0;
+  evaluate<double>([&](auto &ar) {
+    double cf[2];
+    fast_speeds<double>(ar, w, gamma, cf);
+    v1 = fabs(w[0]) + cf[0];
+    v2 = fabs(w[1]) + cf[1];
+  });
+  // neither speed is negative: their bits are in their order, a NaN (its sign
+  // taken off) above all
+  auto bits = [](double v) {
+    return bits_nan(v) ? 0x7ff8000000000000ull : static_cast<unsigned long long>(__double_as_longlong(v));
+  };
+  const unsigned long long b1 = bits(v1), b2 = bits(v2);
+  unsigned long long m = b1 > b2 ? b1 : b2;
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_xor_sync(0xffffffffu, m, o);
-    m = v < m ? v : m;
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+    m = v > m ? v : m;
   }
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double mm = red[0];
-    for (int q = 1; q < static_cast<int>(blockDim.x >> 5); q++) mm = red[q] < mm ? red[q] : mm;
-    *out = nan ? NAN : mm;
-  }
+  if (threadIdx.x != 0) return;
+  for (int q = 1; q < 8; q++) m = red[q] > m ? red[q] : m;
+  const double v = smin(dxdy[2 * blockIdx.x], dxdy[2 * blockIdx.x + 1]) / __longlong_as_double(static_cast<long long>(m));
+  if (isnan(v)) atomicAdd(&g_cfl_nans, 1u);
+  else atomicMin(&g_cfl_key, cfl_key(v));
+  __threadfence();
+  if (atomicAdd(&g_cfl_done, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const unsigned nans = atomicExch(&g_cfl_nans, 0u);
+  const unsigned long long key = atomicExch(&g_cfl_key, kCflKeyMax);
+  g_cfl_done = 0;
+  const double lambda = cfl_unkey(key);
+  *out = nans ? NAN : (key != kCflKeyMax && lambda < 1.E6 ? lambda : 1.E6);
 }
 
 namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
-double *g_scratch_ptr[kMaxDevices] = {nullptr};
+bool g_loaded[kMaxDevices] = {false};
 
-// Set-up of the current device, once per device: the device address of
-// g_cfl_scratch (in host code the symbol is only a stand-in, not a device
-// address), and every kernel of this entry point loaded now (under lazy
-// module loading a kernel first launched inside a stream capture would load
-// there).  The cached address belongs to the device's context: after a
-// cudaDeviceReset it is stale, so this entry point is not used again in that
-// process.
-cudaError_t scratch_for_current_device(double **out) {
+// Every kernel of this entry point loaded on the current device, once: under
+// lazy module loading a kernel first launched inside a stream capture would
+// load there.
+cudaError_t load_on_current_device() {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_mu);
-  if (!g_scratch_ptr[dev]) {
+  if (!g_loaded[dev]) {
     cudaFuncAttributes fa;
-    if ((e = cudaFuncGetAttributes(&fa, k_cfl_static_blocks<2>)) != cudaSuccess) return e;
-    if ((e = cudaFuncGetAttributes(&fa, k_cfl_static_blocks<4>)) != cudaSuccess) return e;
-    if ((e = cudaFuncGetAttributes(&fa, k_cfl_static_min)) != cudaSuccess) return e;
-    void *p = nullptr;
-    e = cudaGetSymbolAddress(&p, g_cfl_scratch);
-    if (e != cudaSuccess) return e;
-    g_scratch_ptr[dev] = static_cast<double *>(p);
+    if ((e = cudaFuncGetAttributes(&fa, k_cfl_static<2>)) != cudaSuccess) return e;
+    if ((e = cudaFuncGetAttributes(&fa, k_cfl_static<4>)) != cudaSuccess) return e;
+    g_loaded[dev] = true;
   }
-  *out = g_scratch_ptr[dev];
   return cudaSuccess;
 }
 }  // namespace
@@ -137,12 +130,9 @@ extern "C" int amr_cfl_dt_static(const double *U, int32_t nblocks, int32_t nghos
   // an error the caller's own earlier work left pending is theirs: report
   // it without clearing it, and launch nothing
   if (cudaPeekAtLastError() != cudaSuccess) return AMR_E_CUDA;
-  double *scratch = nullptr;
-  if (scratch_for_current_device(&scratch) != cudaSuccess) return AMR_E_CUDA;
+  if (load_on_current_device() != cudaSuccess) return AMR_E_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (nghosts == 2) k_cfl_static_blocks<2><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, scratch);
-  else k_cfl_static_blocks<4><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, scratch);
-  if (cudaGetLastError() != cudaSuccess) return AMR_E_CUDA;
-  k_cfl_static_min<<<1, 1024, 0, s>>>(scratch, nblocks, dt_per_cfl_out);
+  if (nghosts == 2) k_cfl_static<2><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, dt_per_cfl_out);
+  else k_cfl_static<4><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, dt_per_cfl_out);
   return cudaGetLastError() == cudaSuccess ? AMR_OK : AMR_E_CUDA;
 }

@@ -310,13 +310,12 @@ int amr_adjoint_recorded(amr_handle *h, int32_t *steps);
  *                  of min(dx,dy) / max(|rho| + c_f,x, |u| + c_f,y)); NaN if a
  *                  block's wave speed is NaN (this variant has no pressure
  *                  trap)
- * The per-block scratch is a fixed file-scope device array of 65536 doubles
- * (512 KiB on every GPU that loads the library, kept until exit); nblocks
- * above 65536 returns AMR_E_TOO_LARGE.  The first call on a device looks up
- * that array's address and loads the entry point's kernels; make it before
- * any stream capture, and do not use the entry point after a cudaDeviceReset
- * in the same process (the looked-up address belongs to the old context).
- * Calls share the array, so calls that overlap on the GPU (different
+ * The scratch (the running minimum and two counts) is in fixed file-scope
+ * device variables of every GPU that loads the library; nblocks above 65536
+ * returns AMR_E_TOO_LARGE.  The first call on a device loads the entry
+ * point's kernels; make it before any stream capture, and do not use the entry
+ * point after a cudaDeviceReset in the same process.
+ * Calls share the variables, so calls that overlap on the GPU (different
  * streams) race: serialise them on one stream.  An error already pending in
  * the CUDA runtime is reported as AMR_E_CUDA and left for its owner.  Work
  * is enqueued on `cuda_stream`; the call does not synchronise. */

@@ -246,6 +246,17 @@ AMR_HD double scale_pow2(double x, bool &bad) {
   return bits_f64(zero ? h : h + (static_cast<uint32_t>(K) << 20), l);
 }
 
+// x * p for p a power of two, exact, as scale_pow2
+AMR_HD double times_pow2(double x, double p, bool &bad) {
+  const uint64_t u = f64_bits(x);
+  const uint32_t h = static_cast<uint32_t>(u >> 32), l = static_cast<uint32_t>(u);
+  const uint32_t t = h << 1;
+  const bool zero = (t | l) == 0u;
+  const int e = static_cast<int>(t >> 21), k = static_cast<int>((f64_bits(p) >> 52) & 0x7ff) - 1023;
+  bad |= !(zero || (e - 1u < 2046u && e + k - 1u < 2046u));
+  return bits_f64(zero ? h : h + (static_cast<uint32_t>(k) << 20), l);
+}
+
 #ifdef __CUDACC__
 // The arithmetic a formula is evaluated with: the operators of the type, or,
 // for double, the routines above and comparisons and multiplications by
@@ -268,6 +279,7 @@ struct Native {
   __device__ __forceinline__ T quarter(T a) { return T(0.25) * a; }
   __device__ __forceinline__ T twice(T a) { return T(2) * a; }
   __device__ __forceinline__ T quad(T a) { return T(4) * a; }
+  __device__ __forceinline__ T scaled(T a, T p) { return a * p; }   // p a positive power of two
   // comparisons with zero
   __device__ __forceinline__ bool positive(T a) { return a > T(0); }
   __device__ __forceinline__ bool negative(T a) { return a < T(0); }
@@ -288,6 +300,7 @@ struct Soft {
   __device__ __forceinline__ double quarter(double a) { return scale_pow2<-2>(a, bad); }
   __device__ __forceinline__ double twice(double a) { return scale_pow2<1>(a, bad); }
   __device__ __forceinline__ double quad(double a) { return scale_pow2<2>(a, bad); }
+  __device__ __forceinline__ double scaled(double a, double p) { return times_pow2(a, p, bad); }
   // of numbers (a NaN fails in the divisions around them)
   __device__ __forceinline__ bool positive(double a) { return __double_as_longlong(a) > 0; }
   __device__ __forceinline__ bool negative(double a) { return __double_as_longlong(a) < 0 && nonzero(a); }

@@ -179,41 +179,68 @@ __global__ void __launch_bounds__(128, MINB) k_faces_dyn(SplitArgs a) {
   }
 }
 
+// Element r of a block's 8 x NN values in the order of k_resid: first the
+// [LO, HI]^2 cells of the 8 variables, then the others (where the residual is
+// zero), so that a warp is wholly one or the other.  Returns the index k*NN + c.
+template <int NG>
+__device__ __forceinline__ int resid_element(int r, bool &inside) {
+  using G = Geo<NG>;
+  constexpr int N = G::N, NN = G::NN, LO = G::LO, NF = G::NF, IN = NF * NF, OUT = NN - IN, SIDE = N - NF;
+  inside = r < 8 * IN;
+  if (inside) {
+    const int k = r / IN, q = r % IN;
+    return k * NN + (LO + q / NF) * N + LO + q % NF;
+  }
+  const int g = r - 8 * IN, k = g / OUT, q = g % OUT;
+  if (q < LO * N) return k * NN + q;                        // rows below LO
+  if (q < SIDE * N) return k * NN + q + NF * N;             // rows above HI
+  const int m = q - SIDE * N, i = m % SIDE;                 // columns beside [LO, HI]
+  return k * NN + (LO + m / SIDE) * N + (i < LO ? i : i + NF);
+}
+
 // residual on [LO, HI]^2 (zero elsewhere) and the RK stage on every cell
-// (main.cpp:147-157 / 179-189).  Bound by the FP64 pipe; the divisions by
-// cells that are no power of two are Soft (softfp.cuh): 18 and 27 us for the
-// 256 blocks of an Orszag-Tang mesh with four ghost layers, 59 and 71 before.
+// (main.cpp:147-157 / 179-189).  Bound by the FP64 pipe (76-80 % busy): 5 FP64
+// instructions per value in stage 1 and 6 in stage 2, the divisions by the
+// cell size Soft (softfp.cuh) or, for power-of-two cells, on the exponent; a
+// value outside [LO, HI]^2, whose residual is zero, takes none (1 in stage 2).
+// The 256 blocks of an Orszag-Tang mesh with four ghost layers: 15 and 19 us
+// (18 and 27 with every value on the same path; 59 and 71 with the compiler's
+// divisions).
 template <int NG, typename S>
 __global__ void __launch_bounds__(512) k_resid(SplitArgs a) {
   pdl_wait();
   using G = Geo<NG>;
   using T = S;
-  constexpr int N = G::N, NN = G::NN, LO = G::LO, HI = G::HI;
+  constexpr int N = G::N, NN = G::NN;
   const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   // fused fill: the flux fill's snapshots (this kernel writes only qout)
   if (a.fuse.save.nseg) fill_save_all<N, S>(a.fuse, e, static_cast<size_t>(gridDim.x) * blockDim.x);
   if (e >= static_cast<size_t>(a.ntasks) * 8 * NN) return;
-  const int t = static_cast<int>(e / (8 * NN)), r = static_cast<int>(e % (8 * NN));
-  const int c = r % NN;
-  const int i = c % N, j = c / N;
-  const LeafTask task = a.tasks[t];
+  const int t = static_cast<int>(e / (8 * NN));
+  bool inside;
+  const int r = resid_element<NG>(static_cast<int>(e % (8 * NN)), inside);
+  const LeafTask &task = a.tasks[t];
   const size_t idx = static_cast<size_t>(task.slot) * 8 * NN + r;
-  T res = T(0.);
-  if (i >= LO && i <= HI && j >= LO && j <= HI) {
-    const S *ff = static_cast<const S *>(a.ff) + idx;
-    const S *gg = static_cast<const S *>(a.gg) + idx;
-    if (task.inv_dx != 0.0 && task.inv_dy != 0.0)  // power-of-two cells: exact reciprocal
-      res = (ff[1] - ff[0]) * static_cast<T>(task.inv_dx) + (gg[N] - gg[0]) * static_cast<T>(task.inv_dy);
-    else
-      evaluate<T>([&](auto &m) {
-        res = m.div(ff[1] - ff[0], static_cast<T>(task.dx)) + m.div(gg[N] - gg[0], static_cast<T>(task.dy));
-      });
-  }
   const T dt = static_cast<T>(a.inst[task.inst].dt);
   const T q = static_cast<const S *>(a.qin)[idx];
   S *out = static_cast<S *>(a.qout) + idx;
-  if (a.step == 1) *out = q - dt * res;
-  else *out = T(0.5) * (*out + q - dt * res);
+  const T old = a.step == 1 ? T(0) : *out;
+  T d = T(0), v = T(0);   // dt * residual
+  if (inside) {
+    const S *ff = static_cast<const S *>(a.ff) + idx;
+    const S *gg = static_cast<const S *>(a.gg) + idx;
+    const T fx = ff[1] - ff[0], gy = gg[N] - gg[0];
+    if (task.inv_dx != 0.0 && task.inv_dy != 0.0)  // power-of-two cells: exact reciprocal
+      evaluate<T>([&](auto &m) {
+        d = m.scaled(fx, static_cast<T>(task.inv_dx)) + m.scaled(gy, static_cast<T>(task.inv_dy));
+      });
+    else
+      evaluate<T>([&](auto &m) { d = m.div(fx, static_cast<T>(task.dx)) + m.div(gy, static_cast<T>(task.dy)); });
+    d = dt * d;
+  }
+  if (a.step == 1) v = inside ? q - d : q;
+  else evaluate<T>([&](auto &m) { v = m.half(inside ? old + q - d : old + q); });
+  *out = v;
 }
 
 }  // namespace amr

@@ -26,23 +26,33 @@ struct GhostAdjLaunch {
   double *take;            // [nseg][nops][16]: per variable, the op's cell (and its pair)
 };
 
+// segment q, picked with constant indices into the parameter block
+__device__ __forceinline__ GhostSeg adj_seg(const GhostAdjLaunch &g, int q) {
+  GhostSeg s = g.seg[0];
+  if (q == 1) s = g.seg[1];
+  if (q == 2) s = g.seg[2];
+  return s;
+}
+
+// one thread per gather of a segment and variable (blockIdx.y): a loop over
+// the variables in a thread is a chain of loads and stores (20 us for the 20 k
+// gathers of a cell field, 9 so)
 template <int N>
 __global__ void k_ghost_adj_take(GhostAdjLaunch g) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
   if (t >= g.nops * g.nseg) return;
   const int q = t / g.nops, r = t % g.nops;
+  const GhostSeg s = adj_seg(g, q);
+  if (k >= s.nv) return;
   const GhostOp op = g.ops[r];
   if (op.type == GOP_NOP) return;
-  const GhostSeg &s = g.seg[q];
-  double *a = static_cast<double *>(s.field) + static_cast<size_t>(op.dst_slot) * s.nv * (N * N) + op.dst_pos;
+  double *a = static_cast<double *>(s.field) + (static_cast<size_t>(op.dst_slot) * s.nv + k) * (N * N) + op.dst_pos;
   double *out = g.take + (static_cast<size_t>(q) * g.nops + r) * 16;
-  for (int k = 0; k < s.nv; k++) {
-    out[k] = a[k * N * N];
-    a[k * N * N] = 0.0;
-    if (op.type == GOP_COPY2) {  // the pair's second cell
-      out[8 + k] = a[k * N * N + 1];
-      a[k * N * N + 1] = 0.0;
-    }
+  out[k] = a[0];
+  a[0] = 0.0;
+  if (op.type == GOP_COPY2) {  // the pair's second cell
+    out[8 + k] = a[1];
+    a[1] = 0.0;
   }
 }
 
@@ -57,43 +67,43 @@ __device__ __forceinline__ void fine_weights(int kind, int k, double w[4]) {
 template <int N>
 __global__ void k_ghost_adj_give(GhostAdjLaunch g) {
   constexpr int NN = N * N;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
   if (t >= g.nops * g.nseg) return;
   const int q = t / g.nops, r = t % g.nops;
+  const GhostSeg s = adj_seg(g, q);
+  if (k >= s.nv) return;
   const GhostOp op = g.ops[r];
   if (op.type == GOP_NOP) return;
-  const GhostSeg &s = g.seg[q];
   double *fld = static_cast<double *>(s.field);
   const double *in = g.take + (static_cast<size_t>(q) * g.nops + r) * 16;
-  for (int k = 0; k < s.nv; k++) {
-    const double v = in[k];
-    if (op.type == GOP_COPY2) {
-      double *src = fld + (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos;
-      if (v != 0.0) atomicAdd(src, v);
-      if (in[8 + k] != 0.0) atomicAdd(src + 1, in[8 + k]);
-      continue;
-    }
-    if (v == 0.0) continue;
-    if (op.type == GOP_COPY) {
-      atomicAdd(fld + (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos, v);
-    } else if (op.type == GOP_SNAP) {
-      const GhostSnap sn = g.snaps[op.src_slot];
-      atomicAdd(fld + (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos, v);
-    } else {
-      double w[4];
-      fine_weights(s.kind, k, w);
-      for (int p = 0; p < 4; p++) {
-        if (w[p] == 0.0) continue;
-        size_t at;
-        if (op.type == GOP_FINE) {
-          const int off = p == 0 ? 0 : (p == 1 ? N : (p == 2 ? 1 : N + 1));
-          at = (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos + off;
-        } else {  // GOP_SFINE: snapshot rows src_slot .. src_slot + 3
-          const GhostSnap sn = g.snaps[op.src_slot + p];
-          at = (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos;
-        }
-        atomicAdd(fld + at, w[p] * v);
+  const double v = in[k];
+  if (op.type == GOP_COPY2) {
+    double *src = fld + (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos;
+    if (v != 0.0) atomicAdd(src, v);
+    if (in[8 + k] != 0.0) atomicAdd(src + 1, in[8 + k]);
+    return;
+  }
+  if (v == 0.0) return;
+  if (op.type == GOP_COPY) {
+    atomicAdd(fld + (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos, v);
+  } else if (op.type == GOP_SNAP) {
+    const GhostSnap sn = g.snaps[op.src_slot];
+    atomicAdd(fld + (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos, v);
+  } else {
+    double w[4];
+    fine_weights(s.kind, k, w);
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      if (w[p] == 0.0) continue;
+      size_t at;
+      if (op.type == GOP_FINE) {
+        const int off = p == 0 ? 0 : (p == 1 ? N : (p == 2 ? 1 : N + 1));
+        at = (static_cast<size_t>(op.src_slot) * s.nv + k) * NN + op.src_pos + off;
+      } else {  // GOP_SFINE: snapshot rows src_slot .. src_slot + 3
+        const GhostSnap sn = g.snaps[op.src_slot + p];
+        at = (static_cast<size_t>(sn.slot) * s.nv + k) * NN + sn.pos;
       }
+      atomicAdd(fld + at, w[p] * v);
     }
   }
 }
@@ -357,8 +367,9 @@ __device__ __forceinline__ void rusa_adj(M &m, const double *wL, const double *w
 // the residual of the face's two cells) becomes the adjoint of the two
 // reconstructed states, of the normal face field (added to aB) and, through
 // the MUSCL Jacobian, of the primitive state of the four stencil cells (C).
-// Bound by the FP64 pipe; with Soft divisions and roots (softfp.cuh) 303 us
-// for 256 blocks, 387 before.
+// Bound by the FP64 pipe (82 % busy): 233 us for 256 blocks with Soft divisions
+// and roots (softfp.cuh) and fused products and sums; 303 without the fusing,
+// 387 with the compiler's divisions.
 template <int NG, class M>
 __device__ __forceinline__ bool face_adj(const StageAdjArgs &a, size_t e) {
   M ar;

@@ -55,16 +55,7 @@ namespace {
 // instead of 256, as their time is that of one leaf's rounds of cells (196
 // leaves: k_prim_task 13.6 -> 12.6 us, FP32 k_dt_cell 10.3 -> 9.2; 40-leaf
 // Brio-Wu program 6293 -> 6165 us with both)
-bool wide_cta(int ntasks) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 0;
-  }
-  return ntasks <= 2 * sms;
-}
+bool wide_cta(int ntasks) { return ct_coop_pays(ntasks); }
 int cell_threads(const Method &m) { return m.cell_block == 128 || m.cell_block == 512 ? m.cell_block : 256; }
 }  // namespace
 
@@ -143,54 +134,45 @@ cudaError_t launch_ct_face(const Method &m, const CtArgs &a, int n, cudaStream_t
   return AMR_DISPATCH_NG_S_PDL(m, k_ct_face, n, 128, 0, s, a);
 }
 
-// One cooperative launch (all CTAs resident: grid = SMs x resident CTAs per
-// SM, capped at the task count), not a programmatic dependent.  Threads per
-// CTA: a block's phases are rounds of dependent loads, so the widest CTA that
-// still holds every leaf at once wins (512 threads: 456 FP32 or 304 FP64
-// leaves, 256: twice, 128: four times as many), and beyond that 256.  Measured
-// per pass with 128 / 256 / 512 threads (us; one GB300): rotor of 196 leaves
-// FP32 1500 / 1386 / 1281, FP64 1565 / 1515 / 1507; 256 leaves FP64 1487 / 1465
-// / 1459; 1024 leaves FP32 2147 / 2290 / 2212; 3400 leaves FP32 7784 / 7356 /
-// 7600; 6272 leaves FP32 18723 / 18577 / 19538.
 namespace {
-using CtCoopKernel = void (*)(CtArgs, FillFuse, FillFuse, FillFuse, unsigned *);
-struct CtCoop {
-  CtCoopKernel k[3];   // 512, 256, 128 threads
-  int ps[3];           // resident CTAs per SM, looked up once
-};
-template <int NG, typename S>
-CtCoop &ct_coop_of() {
-  static CtCoop c = {{k_ct_coop<NG, S, 512>, k_ct_coop<NG, S, 256>, k_ct_coop<NG, S, 128>}, {0, 0, 0}};
-  return c;
+int sm_count() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 0;
+  }
+  return sms;
 }
 }  // namespace
 
+bool ct_coop_pays(int ntasks) { return ntasks <= 2 * sm_count(); }
+
+// One cooperative launch (all CTAs resident: grid = SMs x resident CTAs per
+// SM, capped at the task count), not a programmatic dependent.  512 threads
+// per CTA: it is taken for few leaves (ct_coop_pays), whose phases are rounds
+// of dependent loads (rotor of 196 leaves, us per pass with 128 / 256 / 512
+// threads: FP32 1500 / 1386 / 1281, FP64 1565 / 1515 / 1507).
 cudaError_t launch_ct_coop(const Method &m, const CtArgs &a, const FillFuse &f_emf, const FillFuse &f_face,
                            const FillFuse &f_cell, unsigned *bar, cudaStream_t s) {
   if (a.ntasks <= 0) return cudaSuccess;
-  static int sms = 0;
-  CtCoop &c = m.ng == 2 ? (m.f32 ? ct_coop_of<2, float>() : ct_coop_of<2, double>())
-                        : (m.f32 ? ct_coop_of<4, float>() : ct_coop_of<4, double>());
-  if (!sms) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  static int per_sm[2][2] = {{0, 0}, {0, 0}};
+  constexpr int threads = 512;
+  void (*k)(CtArgs, FillFuse, FillFuse, FillFuse, unsigned *) =
+      m.ng == 2 ? (m.f32 ? k_ct_coop<2, float, threads> : k_ct_coop<2, double, threads>)
+                : (m.f32 ? k_ct_coop<4, float, threads> : k_ct_coop<4, double, threads>);
+  int &ps = per_sm[m.ng == 2 ? 0 : 1][m.f32 ? 1 : 0];
+  if (!ps) {
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k, threads, 0);
     if (e != cudaSuccess) return e;
+    if (ps < 1) return cudaErrorInvalidConfiguration;
   }
-  int pick = -1;
-  for (int q = 0; q < 3; q++) {
-    if (!c.ps[q]) {
-      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.ps[q], c.k[q], 512 >> q, 0);
-      if (e != cudaSuccess) return e;
-      if (c.ps[q] < 1) return cudaErrorInvalidConfiguration;
-    }
-    if (pick < 0 && a.ntasks <= sms * c.ps[q]) pick = q;
-  }
-  if (pick < 0) pick = 1;
-  const int cap = sms * c.ps[pick];
+  const int cap = sm_count() * ps;
+  if (cap < 1) return cudaErrorInvalidDevice;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.ntasks < cap ? a.ntasks : cap);
-  cfg.blockDim = dim3(512 >> pick);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
@@ -198,7 +180,7 @@ cudaError_t launch_ct_coop(const Method &m, const CtArgs &a, const FillFuse &f_e
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, c.k[pick], a, f_emf, f_face, f_cell, bar);
+  return cudaLaunchKernelEx(&cfg, k, a, f_emf, f_face, f_cell, bar);
 }
 
 cudaError_t launch_diffuse(const Method &m, const CtArgs &a, int n, cudaStream_t s) {

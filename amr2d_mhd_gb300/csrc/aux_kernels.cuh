@@ -123,6 +123,12 @@ __device__ __forceinline__ void ct_emf_upwind(const CtArgs &a, const LeafTask &t
   }
 }
 
+__device__ __forceinline__ double widened(double x) { return x; }
+__device__ __forceinline__ double widened(float x) { return to_f64(x); }
+// half of a face sum in the storage type (halving is exact)
+__device__ __forceinline__ double half_as(double sum, double) { return 0.5 * sum; }
+__device__ __forceinline__ float half_as(double sum, float) { return 0.5f * to_f32(sum); }
+
 // CT2D.cpp:16-26 corner EMF for i, j in [1, N), block of task t (sp, sC:
 // shared scratch of the upwind form)
 template <int NG, typename S>
@@ -146,7 +152,7 @@ __device__ __forceinline__ void ct_emf_block(const CtArgs &a, const FillFuse &f,
     // round-off whatever the EMF's precision)
     const S g5a = gg[5 * NN + j * N + i - 1], g5b = gg[5 * NN + c];
     const S f6a = ff[6 * NN + (j - 1) * N + i], f6b = ff[6 * NN + c];
-    E[c] = static_cast<double>(S(0.25) * ((g5a + g5b) - (f6a + f6b)));
+    E[c] = widened(S(0.25) * ((g5a + g5b) - (f6a + f6b)));
   }
   fuse_save<N, S>(f, t);
 }
@@ -156,19 +162,25 @@ template <int NG, typename S>
 __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f, const LeafTask &t) {
   constexpr int N = Geo<NG>::N, NN = N * N;
   fuse_apply<N, S>(f, t);
-  const double dt = a.inst[t.inst].dt;
+  const double dt = a.inst[t.inst].dt, part = a.step == 1 ? 1.0 : 0.5;
   const double *E = a.EMF + static_cast<size_t>(t.slot) * NN;
   const double *B0 = a.Bsrc + static_cast<size_t>(t.slot) * 2 * NN;
   double *B1 = a.Bnew + static_cast<size_t>(t.slot) * 2 * NN;
   for (int c = block_tid(); c < NN; c += blockDim.x) {
     const int i = c % N, j = c / N;
     const int ip = i < N - 1 ? i + 1 : i, jp = j < N - 1 ? j + 1 : j;
-    double res = t.rcp_dy * (E[jp * N + i] - E[c]);
-    if (a.step == 1) B1[c] = B0[c] - dt * res;
-    else B1[c] = 0.5 * (B0[c] + B1[c] - dt * res);
-    res = -t.rcp_dx * (E[j * N + ip] - E[c]);
-    if (a.step == 1) B1[NN + c] = B0[NN + c] - dt * res;
-    else B1[NN + c] = 0.5 * (B0[NN + c] + B1[NN + c] - dt * res);
+    // products and halvings on the integer pipe: as FP64 instructions they
+    // were most of the pipe's work, which bound this kernel in batches (6272
+    // FP32 leaves, predictor and corrector: 58 and 84 us before, 50 and 51 now)
+    const double e0 = E[c], ey = E[jp * N + i] - e0, ex = e0 - E[j * N + ip];   // ex: minus the reference's
+    double bx = B0[c], by = B0[NN + c], nx = 0, ny = 0;
+    if (a.step != 1) { bx += B1[c]; by += B1[NN + c]; }
+    evaluate<double>([&](auto &m) {
+      nx = m.scaled(bx - m.mul(dt, m.mul(t.rcp_dy, ey)), part);
+      ny = m.scaled(by - m.mul(dt, m.mul(t.rcp_dx, ex)), part);
+    });
+    B1[c] = nx;
+    B1[NN + c] = ny;
   }
   fuse_save<N, S>(f, t);
 }
@@ -187,8 +199,8 @@ __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f
     const int jp = j < N - 1 ? j + 1 : j, jj = jp - 1;
     // face averages from the FP64 face field, rounded once to the storage
     // type; the energy correction in the storage type (FP64 on the FP64 path)
-    const S bx = static_cast<S>(0.5 * (B[j * N + ip] + B[j * N + ii]));
-    const S by = static_cast<S>(0.5 * (B[NN + jp * N + i] + B[NN + jj * N + i]));
+    const S bx = half_as(B[j * N + ip] + B[j * N + ii], S(0));
+    const S by = half_as(B[NN + jp * N + i] + B[NN + jj * N + i], S(0));
     const S q5 = q[5 * NN + c], q6 = q[6 * NN + c];
     q[4 * NN + c] = q[4 * NN + c] + S(0.5) * ((bx * bx + by * by) - (q5 * q5 + q6 * q6));
     q[5 * NN + c] = bx;
@@ -197,8 +209,13 @@ __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f
   fuse_save<N, S>(f, t);
 }
 
+// The three kernels of CT2D for many leaves (launch.hpp, ct_coop_pays), one
+// leaf per CTA.  The EMF and cell kernels wait for the loads of their fills'
+// gathers, so registers are held to 40 (64) for 12 (8) CTAs per SM; 6272 FP32
+// leaves: EMF 121, cells 52 us before and 40 now, with the conversions to and
+// from FP32 off the FP64 pipe.
 template <int NG, typename S>
-__global__ void k_ct_emf(CtArgs a) {
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_emf(CtArgs a) {
   pdl_wait();
   constexpr int NN = Geo<NG>::NN;
   __shared__ S sp[NN], sC[NN];
@@ -206,13 +223,13 @@ __global__ void k_ct_emf(CtArgs a) {
 }
 
 template <int NG, typename S>
-__global__ void k_ct_face(CtArgs a) {
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_face(CtArgs a) {
   pdl_wait();
   ct_face_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x]);
 }
 
 template <int NG, typename S>
-__global__ void k_ct_cell(CtArgs a) {
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_cell(CtArgs a) {
   pdl_wait();
   ct_cell_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x]);
 }
@@ -256,12 +273,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, DevError *err) {
 // snapshots saved by the phase before.  The EMF phase also gathers the fill
 // of the fluxes and face field that precedes CT2D (main.cpp:161-163), and
 // the cell phase saves the snapshots of the cell fill that follows it.  Bound
-// by the latency of the gathers: with groups of variables per thread and wide
-// CTAs for few leaves (launch_ct_coop) 6272 FP32 leaves take 240 us (268
-// before), 196 take 23 (33), 196 FP64 leaves 26 (37).  Registers are held to 40
-// (FP32) and 64 for the resident warps.
+// by the latency of the gathers: with groups of variables per thread and 512
+// threads per CTA 196 FP32 leaves take 23 us (33 before), 196 FP64 leaves 26 (37).
 template <int NG, typename S, int THREADS>
-__global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1536 : 1024) / THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
                                                      unsigned *bar) {
   pdl_wait();
   constexpr int NN = Geo<NG>::NN;
@@ -397,7 +412,7 @@ __device__ __forceinline__ void dt_cell(const DtArgs &a) {
     T lamT = T(0.);
     evaluate<T>([&](auto &m) {
       T cf[2];
-      fast_speeds<T>(m, w, g, cf);
+      fast_speeds_of(m, w, g, cf);
       lamT = smax(fabs(w[0]) + cf[0], fabs(w[1]) + cf[1]);
     });
     const double lam = static_cast<double>(warp_max_t(lamT));

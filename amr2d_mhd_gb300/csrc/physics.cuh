@@ -233,12 +233,13 @@ __device__ __forceinline__ T fast_speed(M &m, const T *w, T gamma, int norm) {
 }
 
 // FP32 faces: the squares of the sound and Alfven speeds as they are, without
-// the roots that the FP64 path takes and squares again (fewer roundings)
-__device__ __forceinline__ float fast_speed_of(Quick &m, const float *w, float gamma, float b2) {
+// the roots that the FP64 path takes and squares again, and the transverse
+// field's share as a sum instead of a difference (fewer roundings, and never negative)
+__device__ __forceinline__ float fast_speed_of(Quick &m, const float *w, float gamma) {
   const float ir = m.div(1.f, w[0]);
-  const float c2 = b2 * ir, a2 = gamma * w[4] * ir, n2 = w[5] * w[5] * ir;
+  const float t2 = (w[6] * w[6] + w[7] * w[7]) * ir, c2 = w[5] * w[5] * ir + t2, a2 = gamma * w[4] * ir;
   const float d = c2 - a2;
-  return m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (c2 - n2))));
+  return m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * t2)));
 }
 
 // the same for norm 5 (x) and 6 (y), whose first two terms are the same values
@@ -252,6 +253,19 @@ __device__ __forceinline__ void fast_speeds(M &m, const T *w, T gamma, T *cf) {
     const T can = m.root(m.div(w[5 + q] * w[5 + q], w[0]));
     cf[q] = m.root(m.half(i0 + m.root(i1 * i1 + m.quad(a * a) * ((ca * ca) - (can * can)))));
   }
+}
+
+// FP32: as fast_speed_of, with one reciprocal for both
+__device__ __forceinline__ void fast_speeds_of(Native<float> &m, const float *w, float gamma, float *cf) {
+  const float ir = 1.f / w[0];
+  const float bx = w[5] * w[5] * ir, by = w[6] * w[6] * ir, bz = w[7] * w[7] * ir, a2 = gamma * w[4] * ir;
+  const float c2 = bx + by + bz, d = c2 - a2;
+  cf[0] = m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (by + bz))));
+  cf[1] = m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (bx + bz))));
+}
+template <class M>
+__device__ __forceinline__ void fast_speeds_of(M &m, const double *w, double gamma, double *cf) {
+  fast_speeds<double>(m, w, gamma, cf);
 }
 
 // riemannS.cpp:59-108 for one side: the energy, the total pressure and the
@@ -277,7 +291,7 @@ __device__ __forceinline__ void side_scalars(M &m, const T *w, T gamma, T &cf, T
 template <typename T>
 __device__ __forceinline__ void side_scalars(Quick &m, const float *w, float gamma, float &cf, float &pt, float &e) {
   const float b2 = w[5] * w[5] + w[6] * w[6] + w[7] * w[7];
-  cf = fast_speed_of(m, w, gamma, b2);
+  cf = fast_speed_of(m, w, gamma);
   e = m.div(w[4], gamma - 1.f) + 0.5f * (w[0] * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) + b2);
   pt = w[4] + 0.5f * b2;
 }

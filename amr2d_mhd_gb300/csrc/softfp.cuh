@@ -233,6 +233,72 @@ AMR_HD double sqrt_rn(double x, bool &bad) {
   return zero ? x : bits_f64(hi, static_cast<uint32_t>(n));
 }
 
+// a * b, for kernels whose FP64 instructions are few among memory accesses (the
+// CT face update): about 50 integer instructions, 17 clocks per SM and warp
+// beside additions on the FP64 pipe, which takes 20 for a product.  (In the face
+// kernels, which have a quarter of the warps in flight to hide those 50
+// instructions, products stayed faster on the FP64 pipe.)
+AMR_HD double mul_rn(double a, double b, bool &bad) {
+  const uint64_t ua = f64_bits(a), ub = f64_bits(b);
+  const uint32_t ah = static_cast<uint32_t>(ua >> 32), al = static_cast<uint32_t>(ua);
+  const uint32_t bh = static_cast<uint32_t>(ub >> 32), bl = static_cast<uint32_t>(ub);
+  const uint32_t ea = ah & 0x7ff00000u, eb = bh & 0x7ff00000u;
+  // a zero operand, or exponents so small together that the product, below 2^-1075, rounds to zero
+  const bool za = ((ah << 1) | al) == 0u, zb = ((bh << 1) | bl) == 0u;
+  const bool zero = za || zb || ea + eb <= (969u << 20);
+  // normal operands and a result exponent inside the normal range, or zeros and normal operands
+  const uint32_t er = ea + eb - (1024u << 20);   // (exponent of the product) - 1, if it is not doubled
+  bad |= !((za || ea - (1u << 20) < (2046u << 20)) && (zb || eb - (1u << 20) < (2046u << 20)) &&
+           (zero || er < (2044u << 20)));
+  // the 106-bit product of the significands: h 2^64 + (low word of c) 2^32 + (low word of p)
+  const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t p = static_cast<uint64_t>(al) * bl;
+  const uint64_t c = static_cast<uint64_t>(al) * mbh + (static_cast<uint64_t>(mah) * bl + (p >> 32));
+  const uint64_t h = static_cast<uint64_t>(mah) * mbh + (c >> 32);
+  const uint32_t hh = static_cast<uint32_t>(h >> 32), hl = static_cast<uint32_t>(h), w = static_cast<uint32_t>(c);
+  const uint32_t top = hh >> 9;                  // 1 if the product is in [2, 4)
+  const int s = 12 - static_cast<int>(top);
+  const uint32_t nl = shl_hi(w, hl, s), nh = shl_hi(hl, hh, s);
+  // what is cut off, its last bit standing for everything below; round to nearest even
+  const uint32_t rest = (w << s) | (static_cast<uint32_t>(p) != 0u ? 1u : 0u);
+  const uint32_t up = static_cast<uint32_t>((static_cast<uint64_t>(rest) + 0x7fffffffu + (nl & 1u)) >> 32);
+  const uint64_t n = ((static_cast<uint64_t>(nh) << 32) | nl) + up;
+  const uint32_t hi = static_cast<uint32_t>(n >> 32) + er + (top << 20);
+  const uint32_t sign = (ah ^ bh) & 0x80000000u;
+  return bits_f64((zero ? 0u : hi) | sign, zero ? 0u : static_cast<uint32_t>(n));
+}
+
+// double to float (to nearest even) and back on the integer pipe, where the
+// conversion instructions take the FP64 pipe; outside the float's normal range
+// the conversion itself
+AMR_HD float to_f32(double x) {
+  const uint64_t u = f64_bits(x);
+  const uint32_t h = static_cast<uint32_t>(u >> 32), l = static_cast<uint32_t>(u);
+  const uint32_t e = (h >> 20) & 0x7ffu;
+  if ((h << 1 | l) != 0u && e - 897u >= 253u) return static_cast<float>(x);
+  const uint32_t m = shl_hi(l, h & 0xfffffu, 3);
+  const uint32_t up = static_cast<uint32_t>((static_cast<uint64_t>(l << 3) + 0x7fffffffu + (m & 1u)) >> 32);
+  const uint32_t b = (h & 0x80000000u) | ((h << 1 | l) == 0u ? 0u : ((e - 896u) << 23) + m + up);
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(b);
+#else
+  float f;
+  memcpy(&f, &b, 4);
+  return f;
+#endif
+}
+AMR_HD double to_f64(float x) {
+#ifdef __CUDA_ARCH__
+  const uint32_t b = __float_as_uint(x);
+#else
+  uint32_t b;
+  memcpy(&b, &x, 4);
+#endif
+  const uint32_t e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
+  if ((b << 1) != 0u && e - 1u >= 254u) return static_cast<double>(x);
+  return (b << 1) == 0u ? bits_f64(b, 0u) : bits_f64((b & 0x80000000u) | ((e + 896u) << 20) | (m >> 3), m << 29);
+}
+
 // 2^K x, exact: the exponent field moved, zeros kept.  A result or operand
 // outside the normal range sets `bad`.
 template <int K>
@@ -269,6 +335,7 @@ struct Native {
   __device__ __forceinline__ T div(T a, T b) { return a / b; }
   __device__ __forceinline__ T root(T x) { return sqrt(x); }
   template <int B> __device__ __forceinline__ T by(T a) { return a / T(B); }
+  __device__ __forceinline__ T mul(T a, T b) { return a * b; }
   // the larger of two values that are not negative; Soft compares the bits,
   // where a NaN counts as the largest (and the division it reaches fails)
   __device__ __forceinline__ T most(T a, T b) { return a > b ? a : b; }
@@ -293,6 +360,7 @@ struct Soft {
   __device__ __forceinline__ double div(double a, double b) { return div_rn(a, b, bad); }
   __device__ __forceinline__ double root(double x) { return sqrt_rn(x, bad); }
   template <int B> __device__ __forceinline__ double by(double a) { return div_by<B>(a, bad); }
+  __device__ __forceinline__ double mul(double a, double b) { return mul_rn(a, b, bad); }
   __device__ __forceinline__ double most(double a, double b) { return f64_bits(a) > f64_bits(b) ? a : b; }
   __device__ __forceinline__ double std_most(double a, double b) { return most(a, b); }
   __device__ __forceinline__ double least(double a, double b) { return f64_bits(a) < f64_bits(b) ? a : b; }
@@ -337,8 +405,13 @@ __device__ __forceinline__ void evaluate(F &&f) {
   typename ArithOf<T>::type m;
   f(m);
   if (m.failed()) {
+    // as a loop (of one round), which stays a branch: a short body would be
+    // predicated, and its FP64 instructions issued to the pipe all the same
+    // (k_ct_face, 6272 leaves: 55 us predicated, 42 with the branch)
     Native<T> n;
-    f(n);
+    int rounds = 1;
+    asm volatile("" : "+r"(rounds));
+    for (; rounds > 0; rounds--) f(n);
   }
 }
 #endif

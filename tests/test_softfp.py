@@ -90,6 +90,36 @@ def test_soft_division_and_root_on_the_gpu(gpu):
         compare(L, 1 << 20, seed)
 
 
+def compare_mul(L, n, seed):
+    """Products and the conversions between double and float, bit for bit."""
+    a, b = operands(n, seed)
+    g = np.random.default_rng(seed + 1)
+    few = g.random(n) < 0.3   # on float's grid and halfway between its values
+    a[few] = (a[few].view(np.int64) & ~np.int64((1 << 28) - 1)).view(np.float64)
+    out, bad = np.zeros((3, n)), np.zeros(n, np.uint8)
+    L.softmul_check.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_long, ctypes.c_void_p, ctypes.c_void_p]
+    assert L.softmul_check(a.ctypes.data, b.ctypes.data, n, out.ctypes.data, bad.ctypes.data) == 0
+    ok = bad == 0
+    with np.errstate(all="ignore"):
+        p, f = a * b, a.astype(np.float32).astype(np.float64)
+        mid = (np.abs(a) > 1e-150) & (np.abs(a) < 1e150) & (np.abs(b) > 1e-150) & (np.abs(b) < 1e150)
+    assert np.array_equal(out[0][ok].view(np.int64), p[ok].view(np.int64))
+    assert ok[mid].all() and ok[(a == 0) & np.isfinite(b) & (np.abs(b) > 1e-300)].all()
+    for o in out[1:]:
+        nan = np.isnan(f)
+        assert np.array_equal(np.isnan(o), nan) and np.array_equal(o[~nan].view(np.int64), f[~nan].view(np.int64))
+
+
+def test_soft_product_and_conversions_on_the_cpu():
+    compare_mul(check_lib(False), 1 << 20, 21)
+
+
+@pytest.mark.gpu
+def test_soft_product_and_conversions_on_the_gpu(gpu):
+    for seed in range(30, 34):
+        compare_mul(check_lib(True), 1 << 20, seed)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("flux", ["RUSA", "HLLE", "HLLC", "HLLD"])
 def test_riemann_with_operands_outside_the_soft_range(gpu, flux):

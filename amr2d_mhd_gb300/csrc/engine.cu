@@ -79,7 +79,7 @@ Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (void *p : {U_, Us_, ff_, gg_, W_}) if (p) cudaFree(p);
   for (double *p : {Bi_, Bis_, EMF_}) if (p) cudaFree(p);
-  for (DevBuf *b : {&d_tasks_, &d_params_, &d_lambda_, &d_grad_, &d_err_, &d_snap_, &d_treeops_, &d_stage_,
+  for (DevBuf *b : {&d_tasks_, &d_params_, &d_grad_, &d_snap_, &d_treeops_, &d_stage_,
                     &d_ctr_, &d_snap3_, &d_bar_})
     b->release();
   d_ops_.release();
@@ -198,13 +198,12 @@ int Engine::create(const amr_config *cfgs, int n) {
     in.slot.assign(in.tree.maxblocks(), -1);
   }
   built_version_.assign(n, ~0ull);
-  CK(d_err_.ensure(sizeof(DevError)), "alloc");
-  CK(cudaMemsetAsync(d_err_.p, 0, sizeof(DevError), stream_), "memset");
   CK(d_ctr_.ensure(2 * sizeof(unsigned)), "alloc");   // k_faces_dyn's counters, zero between launches
   CK(cudaMemsetAsync(d_ctr_.p, 0, 2 * sizeof(unsigned), stream_), "memset");
   CK(d_bar_.ensure(2 * sizeof(unsigned)), "alloc");   // k_ct_coop's grid barrier (count, generation)
   CK(cudaMemsetAsync(d_bar_.p, 0, 2 * sizeof(unsigned), stream_), "memset");
   CK(h_err_.ensure(sizeof(DevError)), "alloc");
+  std::memset(h_err_.p, 0, sizeof(DevError));
   CK(h_params_.ensure(sizeof(InstParams) * n), "alloc");
   CK(d_params_.ensure(sizeof(InstParams) * n), "alloc");
   return AMR_OK;
@@ -503,8 +502,6 @@ int Engine::rebuild() {
   CK(h_tasks_.ensure(sizeof(LeafTask) * nt), "alloc");
   std::memcpy(h_tasks_.p, tasks_.data(), sizeof(LeafTask) * nt);
   CK(cudaMemcpyAsync(d_tasks_.p, h_tasks_.p, sizeof(LeafTask) * nt, cudaMemcpyHostToDevice, stream_), "h2d");
-  CK(d_lambda_.ensure(sizeof(double) * nt), "alloc");
-  CK(d_grad_.ensure(sizeof(double) * nt), "alloc");
   CK(h_lambda_.ensure(sizeof(double) * nt), "alloc");
   CK(h_grad_.ensure(sizeof(double) * nt), "alloc");
   // the pinned mirrors above must not change before the copies have run
@@ -584,7 +581,7 @@ FillFuse Engine::fill_fuse(const FillPass *apply, const FillPass *save) const {
   return f;
 }
 
-int Engine::snap_only(const FillPass &p) {
+int Engine::snap_only(const FillPass &p, bool params) {
   if (nsnaps_ == 0) return AMR_OK;
   GhostLaunch g{};
   g.ops = d_ops_.as<GhostOp>();
@@ -594,6 +591,12 @@ int Engine::snap_only(const FillPass &p) {
   for (int q = 0; q < p.nseg; q++) g.seg[q] = p.seg[q];
   g.nseg = p.nseg;
   g.snapbuf = p.snapbuf;
+  if (params) {
+    g.params_from = h_params_.as<InstParams>();
+    g.params_to = d_params_.as<InstParams>();
+    g.nparams = static_cast<int>(inst_.size());
+    prof_.h2d_bytes += static_cast<int64_t>(sizeof(InstParams) * inst_.size());
+  }
   CK(launch_ghost(m_, g, stream_), "ghost snapshots");
   prof_.launches += 1;
   return AMR_OK;
@@ -630,7 +633,7 @@ int Engine::stage(int step, const FillFuse *fuse) {
     a.B = step == 1 ? Bi_ : Bis_;
     a.ff = ff_;
     a.gg = gg_;
-    a.err = d_err_.as<DevError>();
+    a.err = h_err_.as<DevError>();
     a.ctr = d_ctr_.as<unsigned>();
     a.step = step;
     a.ntasks = n;
@@ -650,7 +653,7 @@ int Engine::stage(int step, const FillFuse *fuse) {
     a.B = step == 1 ? Bi_ : Bis_;
     a.ff = ff_;
     a.gg = gg_;
-    a.err = d_err_.as<DevError>();
+    a.err = h_err_.as<DevError>();
     a.ctr = d_ctr_.as<unsigned>();
     a.step = step;
     a.ntasks = n;
@@ -771,7 +774,7 @@ int Engine::ct2d(int step, const FillPass *in, const FillPass *out, int emf_buf,
   a.Bsrc = step == 1 ? Bi_ : Bis_;
   a.Bnew = step == 1 ? Bis_ : Bi_;
   a.q = step == 1 ? Us_ : U_;
-  a.err = d_err_.as<DevError>();
+  a.err = h_err_.as<DevError>();
   a.step = step;
   const int n = static_cast<int>(tasks_.size());
   a.ntasks = n;
@@ -809,9 +812,9 @@ int Engine::dt_crit(bool want_grad, const FillFuse *fuse) {
   a.tasks = d_tasks_.as<LeafTask>();
   a.inst = d_params_.as<InstParams>();
   a.U = U_;
-  a.lambda = d_lambda_.as<double>();
-  a.grad = d_grad_.as<double>();
-  a.err = d_err_.as<DevError>();
+  a.lambda = h_lambda_.as<double>();
+  a.grad = h_grad_.as<double>();
+  a.err = h_err_.as<DevError>();
   a.want_grad = want_grad ? 1 : 0;
   if (fuse) a.fuse = *fuse;
   CK(launch_dt_cell(m_, a, static_cast<int>(tasks_.size()), stream_), "dt kernel");
@@ -833,7 +836,7 @@ int Engine::enqueue_stage_sequence() {
     const FillPass f5 = fill_pass({{FILL_CC, AMR_FIELD_US}}, 1, 0);
     const FillPass f6 = fill_pass({{FILL_FC, AMR_FIELD_FF}, {FILL_FC, AMR_FIELD_GG}}, 2);
     const FillPass f9 = fill_pass({{FILL_CC, AMR_FIELD_U}}, 2);
-    if ((rc = snap_only(f1))) return rc;
+    if ((rc = snap_only(f1, true))) return rc;
     const FillFuse s1 = fill_fuse(&f1, &f2);
     if ((rc = stage(1, &s1))) return rc;
     if ((rc = ct2d(1, &f2, &f5, 2, 0))) return rc;     // EMF fill in buffer 2, Bis fill in 0
@@ -857,15 +860,13 @@ int Engine::enqueue_stage_sequence() {
 }
 
 int Engine::enqueue_step() {
-  if (int rc = upload_params()) return rc;
+  const bool with_snap = fused_fills() && nsnaps_ != 0;   // else the parameters are a copy of their own
+  if (with_snap) fill_params_host();
+  else if (int rc = upload_params()) return rc;
   if (int rc = enqueue_stage_sequence()) return rc;
   bool any_amr = false;
   for (int a : active_) any_amr |= inst_[a].cfg.maxlevs > 1;
-  if (int rc = dt_crit(any_amr, dt_fuse_.apply.nseg ? &dt_fuse_ : nullptr)) return rc;
-  const size_t nt = tasks_.size();
-  CK(cudaMemcpyAsync(h_lambda_.p, d_lambda_.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, stream_), "d2h");
-  CK(cudaMemcpyAsync(h_grad_.p, d_grad_.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, stream_), "d2h");
-  return AMR_OK;
+  return dt_crit(any_amr, dt_fuse_.apply.nseg ? &dt_fuse_ : nullptr);
 }
 
 int Engine::launch_step() {
@@ -929,7 +930,7 @@ int Engine::launch_step_work() {
     graph_launches_ = prof_.launches - launches0;
     prof_.host_capture_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   } else {
-    fill_params_host();  // the graph's first node copies these to the device
+    fill_params_host();  // the graph's first kernel takes these to the device
     prof_.launches += graph_launches_;
     prof_.stage_launches += 2;
     stage_cells_pending_ += 2 * static_cast<int64_t>(tasks_.size()) * NI * NI;
@@ -941,8 +942,6 @@ int Engine::launch_step_work() {
 }
 
 int Engine::check_device_error() {
-  CK(cudaMemcpyAsync(h_err_.p, d_err_.p, sizeof(DevError), cudaMemcpyDeviceToHost, stream_), "d2h");
-  prof_.d2h_bytes += sizeof(DevError);
   const auto w0 = std::chrono::steady_clock::now();
   CK(cudaStreamSynchronize(stream_), "sync");
   prof_.wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();

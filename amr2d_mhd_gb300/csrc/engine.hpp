@@ -149,7 +149,7 @@ class Engine {
   // fused fills: a fill of `what` with its snapshots in rotating buffer `buf`
   FillPass fill_pass(std::initializer_list<std::pair<FillKind, int>> what, int buf, int tile_seg = -1);
   FillFuse fill_fuse(const FillPass *apply, const FillPass *save) const;
-  int snap_only(const FillPass &p);    // a fill's snapshot pass as a launch of its own
+  int snap_only(const FillPass &p, bool params = false);   // a fill's snapshot pass as a launch of its own, with the parameters' upload
   bool fused_fills() const { return fuse_fills_ && fuse_ok_; }
   int finish_step();
   struct AdmeshMarks {
@@ -198,7 +198,7 @@ class Engine {
   int64_t nops_ = 0, nsnaps_ = 0, hole_ops_ = 0;
   int compile_programs();          // recompile changed instances (host threads)
   int layout_programs(bool relayout);
-  DevBuf d_tasks_, d_params_, d_lambda_, d_grad_, d_err_, d_snap_, d_ops_, d_snaps_;
+  DevBuf d_tasks_, d_params_, d_grad_, d_snap_, d_ops_, d_snaps_;
   DevBuf d_treeops_, d_stage_, d_ctr_;
   DevBuf d_snap3_;                 // fused fills: three rotating snapshot buffers
   DevBuf d_bar_;                   // grid barrier of the cooperative CT launch

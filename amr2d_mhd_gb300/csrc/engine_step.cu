@@ -147,7 +147,7 @@ int Engine::admesh_all(const std::vector<int> &which, const std::vector<std::vec
   a.inst = d_params_.as<InstParams>();
   a.U = U_;
   a.Bi = Bi_;
-  a.err = d_err_.as<DevError>();
+  a.err = h_err_.as<DevError>();
   CK(launch_refine(m_, a, static_cast<int>(ref.size()), stream_), "refine");
   a.ops = d_treeops_.as<TreeOp>() + ref.size();
   CK(launch_coarsen(m_, a, static_cast<int>(crs.size()), stream_), "coarsen");
@@ -360,8 +360,6 @@ int Engine::api_cfl_dt(double *lambda_min) {
   if (int rc = upload_params()) return rc;
   if (int rc = dt_crit(true)) return rc;
   const size_t nt = tasks_.size();
-  CK(cudaMemcpyAsync(h_lambda_.p, d_lambda_.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, stream_), "d2h");
-  CK(cudaMemcpyAsync(h_grad_.p, d_grad_.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, stream_), "d2h");
   if (int rc = check_device_error()) return rc;
   double lambda = 1.E6;
   for (size_t t = 0; t < nt; t++) {

@@ -31,6 +31,11 @@ struct GhostLaunch {
   // variable rows of the launch: segment q owns rows [row0[q], row0[q+1]);
   // set by launch_ghost
   int row0[kMaxSeg + 1];
+  // the snapshots that begin a step also take its parameters from pinned host
+  // memory to the device (nparams 0: not)
+  const InstParams *params_from;
+  InstParams *params_to;
+  int nparams;
 };
 
 // A fill kernel runs on a 2-D grid: blockIdx.y is the variable row, so that

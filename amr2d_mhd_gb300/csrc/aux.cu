@@ -51,11 +51,22 @@ cudaError_t launch_faces(const Method &m, const SplitArgs &a, cudaStream_t s) {
 }
 
 namespace {
+int sm_count() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 0;
+  }
+  return sms;
+}
+
 // Up to two leaves per SM: the kernels with one CTA per leaf take 512 threads
 // instead of 256, as their time is that of one leaf's rounds of cells (196
 // leaves: k_prim_task 13.6 -> 12.6 us, FP32 k_dt_cell 10.3 -> 9.2; 40-leaf
 // Brio-Wu program 6293 -> 6165 us with both)
-bool wide_cta(int ntasks) { return ct_coop_pays(ntasks); }
+bool wide_cta(int ntasks) { return ntasks <= 2 * sm_count(); }
 int cell_threads(const Method &m) { return m.cell_block == 128 || m.cell_block == 512 ? m.cell_block : 256; }
 }  // namespace
 
@@ -124,36 +135,47 @@ cudaError_t launch_ghost(const Method &m, const GhostLaunch &in, cudaStream_t s)
    : !(m).f32                ? launch_k((m).pdl, KERNEL<4, double>, dim3(grid), dim3(block), smem, s, args) \
                              : launch_k((m).pdl, KERNEL<4, float>, dim3(grid), dim3(block), smem, s, args))
 
+namespace {
+// The widest CTAs with which all leaves are resident at once, else 128 threads:
+// the 400 cells of a leaf take 1, 2 or 4 rounds.  KH meshes, us per step with
+// the cooperative launch / 128 / 224 / 416 threads: FP32 16 leaves 79 / - / 76 /
+// 72, 196: 90 / - / 86 / 82.5, 400: 134 / 111 / 104 / 100 (95.5 in a second run,
+// 224: 99.8), 576: - / 121 / 113 / 124, 784: - / 146 / 142 / 149, 1024: 215 / 168
+// / 175 / 179, 4096: 754 / 574 / 589 / 642; FP64 196: 236 / - / 232 / 230, 324:
+// 352 / 343 / 334 / 340, 576: - / 541 / 532 / 539, 784: - / 725 / 729 / 732.
+int ct_threads(const Method &m, int n) {
+  for (const int t : {416, 224})
+    if (n <= sm_count() * (m.f32 ? ct_resident<float>(t) : ct_resident<double>(t))) return t;
+  return 128;
+}
+}  // namespace
+
+#define AMR_CT_WIDTH(m, KERNEL, T, n, s, args)                                                             \
+  (((m).ng == 2 && !(m).f32) ? launch_k((m).pdl, KERNEL<2, double, T>, dim3(n), dim3(T), 0, s, args)       \
+   : ((m).ng == 2)           ? launch_k((m).pdl, KERNEL<2, float, T>, dim3(n), dim3(T), 0, s, args)        \
+   : !(m).f32                ? launch_k((m).pdl, KERNEL<4, double, T>, dim3(n), dim3(T), 0, s, args)       \
+                             : launch_k((m).pdl, KERNEL<4, float, T>, dim3(n), dim3(T), 0, s, args))
+#define AMR_DISPATCH_CT(m, KERNEL, n, s, args)                                       \
+  (ct_threads(m, n) == 416   ? AMR_CT_WIDTH(m, KERNEL, 416, n, s, args)              \
+   : ct_threads(m, n) == 224 ? AMR_CT_WIDTH(m, KERNEL, 224, n, s, args)              \
+                             : AMR_CT_WIDTH(m, KERNEL, 128, n, s, args))
+
+
 cudaError_t launch_ct_emf(const Method &m, const CtArgs &a, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  return AMR_DISPATCH_NG_S_PDL(m, k_ct_emf, n, 128, 0, s, a);
+  return AMR_DISPATCH_CT(m, k_ct_emf, n, s, a);
 }
 
 cudaError_t launch_ct_face(const Method &m, const CtArgs &a, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  return AMR_DISPATCH_NG_S_PDL(m, k_ct_face, n, 128, 0, s, a);
+  return AMR_DISPATCH_CT(m, k_ct_face, n, s, a);
 }
-
-namespace {
-int sm_count() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sms = 0;
-  }
-  return sms;
-}
-}  // namespace
-
-bool ct_coop_pays(int ntasks) { return ntasks <= 2 * sm_count(); }
 
 // One cooperative launch (all CTAs resident: grid = SMs x resident CTAs per
 // SM, capped at the task count), not a programmatic dependent.  512 threads
-// per CTA: it is taken for few leaves (ct_coop_pays), whose phases are rounds
-// of dependent loads (rotor of 196 leaves, us per pass with 128 / 256 / 512
-// threads: FP32 1500 / 1386 / 1281, FP64 1565 / 1515 / 1507).
+// per CTA: the phases of few leaves are rounds of dependent loads (rotor of 196
+// leaves, us per pass with 128 / 256 / 512 threads: FP32 1500 / 1386 / 1281,
+// FP64 1565 / 1515 / 1507).
 cudaError_t launch_ct_coop(const Method &m, const CtArgs &a, const FillFuse &f_emf, const FillFuse &f_face,
                            const FillFuse &f_cell, unsigned *bar, cudaStream_t s) {
   if (a.ntasks <= 0) return cudaSuccess;
@@ -190,7 +212,7 @@ cudaError_t launch_diffuse(const Method &m, const CtArgs &a, int n, cudaStream_t
 
 cudaError_t launch_ct_cell(const Method &m, const CtArgs &a, int n, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  return AMR_DISPATCH_NG_S_PDL(m, k_ct_cell, n, 128, 0, s, a);
+  return AMR_DISPATCH_CT(m, k_ct_cell, n, s, a);
 }
 
 cudaError_t launch_dt_cell(const Method &m, const DtArgs &a, int n, cudaStream_t s) {

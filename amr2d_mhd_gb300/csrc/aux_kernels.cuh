@@ -219,27 +219,31 @@ __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f
   fuse_save<N, S>(f, t);
 }
 
-// The three kernels of CT2D for many leaves (launch.hpp, ct_coop_pays), one
-// leaf per CTA.  The EMF and cell kernels wait for the loads of their fills'
-// gathers, so registers are held to 40 (64) for 12 (8) CTAs per SM; 6272 FP32
-// leaves: EMF 121, cells 52 us before and 40 now, with the conversions to and
-// from FP32 off the FP64 pipe.
-template <int NG, typename S>
-__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_emf(CtArgs a) {
+// The three kernels of CT2D, one leaf per CTA of 416, 224 or 128 threads (the
+// rule at launch_ct_emf in aux.cu).  Few leaves wait for rounds of dependent
+// loads, so wide CTAs; many wait for the loads of their fills' gathers, so
+// registers are held to 40 (64 in FP64) for 1536 (1024) resident threads per SM.
+// 6272 FP32 leaves: EMF 121, faces 50, cells 40 us (121, 58, 52 before the
+// conversions and products left the FP64 pipe).
+template <typename S> __host__ __device__ constexpr int ct_resident(int threads) {
+  return sizeof(S) == 4 ? (threads == 416 ? 3 : (threads == 224 ? 6 : 12)) : (threads == 416 ? 2 : (threads == 224 ? 4 : 8));
+}
+template <int NG, typename S, int THREADS>
+__global__ void __launch_bounds__(THREADS, ct_resident<S>(THREADS)) k_ct_emf(CtArgs a) {
   pdl_wait();
   constexpr int NN = Geo<NG>::NN;
   __shared__ S sp[NN], sC[NN];
   ct_emf_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x], sp, sC);
 }
 
-template <int NG, typename S>
-__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_face(CtArgs a) {
+template <int NG, typename S, int THREADS>
+__global__ void __launch_bounds__(THREADS, ct_resident<S>(THREADS)) k_ct_face(CtArgs a) {
   pdl_wait();
   ct_face_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x]);
 }
 
-template <int NG, typename S>
-__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 12 : 8) k_ct_cell(CtArgs a) {
+template <int NG, typename S, int THREADS>
+__global__ void __launch_bounds__(THREADS, ct_resident<S>(THREADS)) k_ct_cell(CtArgs a) {
   pdl_wait();
   ct_cell_block<NG, S>(a, a.fuse, a.tasks[blockIdx.x]);
 }
@@ -282,9 +286,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, DevError *err) {
 // face field) are fused: gathered by the phase that consumes them, their
 // snapshots saved by the phase before.  The EMF phase also gathers the fill
 // of the fluxes and face field that precedes CT2D (main.cpp:161-163), and
-// the cell phase saves the snapshots of the cell fill that follows it.  Bound
-// by the latency of the gathers: with groups of variables per thread and 512
-// threads per CTA 196 FP32 leaves take 23 us (33 before), 196 FP64 leaves 26 (37).
+// the cell phase saves the snapshots of the cell fill that follows it.  The form
+// with the fewest launches, on request (AMR2D_CT_COOP=1): its barriers cost more
+// than the launches they replace (figures at launch_ct_emf in aux.cu).
 template <int NG, typename S, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_ct_coop(CtArgs a, FillFuse f_emf, FillFuse f_face, FillFuse f_cell,
                                                      unsigned *bar) {

@@ -159,7 +159,7 @@ int Engine::create(const amr_config *cfgs, int n) {
   if (const char *g = std::getenv("AMR2D_GRAPHS")) graph_on_ = std::strcmp(g, "0") != 0;
   if (const char *p = std::getenv("AMR2D_PDL")) m_.pdl = std::strcmp(p, "0") != 0 ? 1 : 0;
   if (const char *f = std::getenv("AMR2D_FUSED_FILLS")) fuse_fills_ = std::strcmp(f, "0") != 0;
-  if (const char *f = std::getenv("AMR2D_CT_COOP")) ct_coop_ = std::strcmp(f, "0") != 0 ? 1 : 0;
+  if (const char *f = std::getenv("AMR2D_CT_COOP")) ct_coop_ = std::strcmp(f, "0") != 0;
   if (const char *f = std::getenv("AMR2D_ZERO_COPY")) zero_copy_ = std::strcmp(f, "0") != 0;
   if (const char *f = std::getenv("AMR2D_FACE_KERNEL"))
     m_.persistent = !std::strcmp(f, "dynamic") ? 2 : (!std::strcmp(f, "persistent") ? 1 : 0);
@@ -781,7 +781,7 @@ int Engine::ct2d(int step, const FillPass *in, const FillPass *out, int emf_buf,
   if (in) {
     const FillPass emf = fill_pass({{FILL_EC, AMR_FIELD_EMF}}, emf_buf);
     const FillPass bnew = fill_pass({{FILL_FC, step == 1 ? AMR_FIELD_BIS : AMR_FIELD_BI}}, bnew_buf);
-    if (ct_coop_ < 0 ? ct_coop_pays(n) : ct_coop_ != 0) {  // one cooperative launch, grid barriers between the phases
+    if (ct_coop_) {  // one cooperative launch, grid barriers between the phases
       CK(launch_ct_coop(m_, a, fill_fuse(in, &emf), fill_fuse(&emf, &bnew), fill_fuse(&bnew, out),
                         d_bar_.as<unsigned>(), stream_), "ct kernel");
       prof_.launches += 1;

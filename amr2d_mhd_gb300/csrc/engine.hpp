@@ -170,7 +170,7 @@ class Engine {
   bool split_ = true;              // stage as prim / faces / resid kernels (else fused k_stage)
   bool fuse_fills_ = true;         // AMR2D_FUSED_FILLS=0: every ghost fill as launches of its own
   bool fuse_ok_ = false;           // every active program is grouped by leaf block
-  int ct_coop_ = -1;               // fused fills: CT2D as one cooperative launch (1, AMR2D_CT_COOP), three (0) or by ct_coop_pays
+  bool ct_coop_ = false;           // fused fills: CT2D as one cooperative launch (AMR2D_CT_COOP=1) instead of three
   // uploads / downloads: the scatter / gather kernel reads / writes the
   // caller's page-locked array itself instead of a copy through a staging
   // buffer (AMR2D_ZERO_COPY=0: always the copy)

@@ -81,13 +81,6 @@ cudaError_t launch_ct_cell(const Method &m, const CtArgs &a, int ntasks, cudaStr
 // the three CT kernels of a stage with fused fills, as one cooperative launch
 // whose phases are separated by grid barriers (bar: two zeroed words)
 struct FillFuse;
-// whether the cooperative launch is the better form: up to two leaves per SM.
-// Beyond, its phases wait for the slowest CTA while three launches keep more
-// warps resident (KH meshes, us per step, cooperative against three launches:
-// 144 leaves FP64 210 / 223, FP32 91 / 97; 256 leaves 294 / 298, 100 / 103; 324
-// leaves 365 / 354, 127 / 115; 1024 leaves 951 / 921, 215 / 182; 4096 leaves
-// 3525 / 3390, 754 / 592)
-bool ct_coop_pays(int ntasks);
 cudaError_t launch_ct_coop(const Method &m, const CtArgs &a, const FillFuse &f_emf, const FillFuse &f_face,
                            const FillFuse &f_cell, unsigned *bar, cudaStream_t s);
 // diffusivity.cpp on the tasks flagged TASK_DIFFUSE (a.q = U after stage 2)

@@ -4,44 +4,52 @@
 // Some hosts cannot call cudaMalloc at the point where they need the time step:
 // code running inside a captured CUDA graph, allocator-free real-time loops,
 // or frameworks that own every device allocation and forbid others.  This
-// entry point takes the caller's device arrays and keeps its only scratch, the
-// running minimum and two counts, in this file's device globals, so it
-// allocates nothing.
+// entry point takes the caller's device arrays and has no scratch: it allocates
+// nothing.
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <mutex>
 
 #include "../../include/amr2d_mhd.h"
+#include "launch.hpp"
 #include "stage.cuh"
 
 namespace amr {
 
 constexpr int kCflStaticMaxBlocks = 1 << 16;
 
-// The minimum over the blocks so far, as a key whose unsigned order is the
-// order of the values, the number of NaN blocks and of finished CTAs; shared
-// by every call.  The last CTA of a launch writes the result and puts the
-// start values back, so a call needs no other launch.
-constexpr unsigned long long kCflKeyMax = ~0ull;
-static __device__ unsigned long long g_cfl_key = kCflKeyMax;
-static __device__ unsigned g_cfl_nans = 0, g_cfl_done = 0;
-
-__device__ __forceinline__ unsigned long long cfl_key(double v) {
-  const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
-  return u >> 63 ? ~u : u | (1ull << 63);
+// The result itself is the running minimum, started at the cap by a launch of
+// its own, so a call depends on nothing that another call has left and calls
+// with results of their own may overlap.
+__global__ void k_cfl_start(double *out) {
+  asm volatile("griddepcontrol.launch_dependents;");   // k_cfl_static waits for this grid before it looks at *out
+  *out = 1.E6;
 }
-__device__ __forceinline__ double cfl_unkey(unsigned long long k) {
-  return __longlong_as_double(static_cast<long long>(k >> 63 ? k & ~(1ull << 63) : ~k));
+
+// *out = min(*out, v), and a NaN for good once v is one.  As bit patterns the
+// values that are not negative order as signed integers, below them the
+// negative ones in reverse as unsigned integers; the NaN taken, all ones, is
+// above every negative value in that second order.
+__device__ __forceinline__ void cfl_take(double *out, double v) {
+  const long long now = *reinterpret_cast<volatile long long *>(out);
+  const long long s = isnan(v) ? -1ll : __double_as_longlong(v);
+  if (s >= 0) {
+    if (s < now) atomicMin(reinterpret_cast<long long *>(out), s);
+  } else if (static_cast<unsigned long long>(s) > static_cast<unsigned long long>(now)) {
+    atomicMax(reinterpret_cast<unsigned long long *>(out), static_cast<unsigned long long>(s));
+  }
 }
 
 // Bound by the FP64 pipe: about 35 FP64 instructions per cell, the divisions
 // and square roots on the integer pipe (softfp.cuh), and the maximum, where a
 // NaN counts as the largest, on the bit patterns.  One thread per interior
-// cell; the minimum over the blocks by an atomic of each CTA, taken over by
-// the last one.  20011 blocks: 0.37 ms (0.72 with a
-// loop over all cells of a block and a second launch for the minimum, 2.25 at
-// first), 64 blocks 9 us (18, 29).
+// cell; the minimum over the blocks by an atomic of each CTA that lowers it.
+// 64 blocks 8.2 us a call, 20011 blocks 370 us.  k_cfl_start beside it costs
+// nothing that shows, as a programmatic dependent is launched while its
+// predecessor runs (the minimum kept in device globals that the last CTA put
+// back, with no second launch: 8.3 and 373 us; the start value by a memset: 9.1
+// and 373).
 //
 // main.cpp:211-228 for one block of the dense array: lambda1 takes |rho| +
 // c_f,x (W[..][0], main.cpp:222) and lambda2 |u| + c_f,y (:224) over the
@@ -83,16 +91,8 @@ __global__ void __launch_bounds__(256) k_cfl_static(const double *U, const doubl
   if (threadIdx.x != 0) return;
   for (int q = 1; q < 8; q++) m = red[q] > m ? red[q] : m;
   const double v = smin(dxdy[2 * blockIdx.x], dxdy[2 * blockIdx.x + 1]) / __longlong_as_double(static_cast<long long>(m));
-  if (isnan(v)) atomicAdd(&g_cfl_nans, 1u);
-  else atomicMin(&g_cfl_key, cfl_key(v));
-  __threadfence();
-  if (atomicAdd(&g_cfl_done, 1u) != gridDim.x - 1) return;
-  __threadfence();
-  const unsigned nans = atomicExch(&g_cfl_nans, 0u);
-  const unsigned long long key = atomicExch(&g_cfl_key, kCflKeyMax);
-  g_cfl_done = 0;
-  const double lambda = cfl_unkey(key);
-  *out = nans ? NAN : (key != kCflKeyMax && lambda < 1.E6 ? lambda : 1.E6);
+  pdl_wait();
+  cfl_take(out, v);
 }
 
 namespace {
@@ -111,6 +111,7 @@ cudaError_t load_on_current_device() {
   std::lock_guard<std::mutex> lock(g_mu);
   if (!g_loaded[dev]) {
     cudaFuncAttributes fa;
+    if ((e = cudaFuncGetAttributes(&fa, k_cfl_start)) != cudaSuccess) return e;
     if ((e = cudaFuncGetAttributes(&fa, k_cfl_static<2>)) != cudaSuccess) return e;
     if ((e = cudaFuncGetAttributes(&fa, k_cfl_static<4>)) != cudaSuccess) return e;
     g_loaded[dev] = true;
@@ -132,7 +133,12 @@ extern "C" int amr_cfl_dt_static(const double *U, int32_t nblocks, int32_t nghos
   if (cudaPeekAtLastError() != cudaSuccess) return AMR_E_CUDA;
   if (load_on_current_device() != cudaSuccess) return AMR_E_CUDA;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (nghosts == 2) k_cfl_static<2><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, dt_per_cfl_out);
-  else k_cfl_static<4><<<nblocks, 256, 0, s>>>(U, dxdy, gamma, dt_per_cfl_out);
-  return cudaGetLastError() == cudaSuccess ? AMR_OK : AMR_E_CUDA;
+  k_cfl_start<<<1, 1, 0, s>>>(dt_per_cfl_out);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_k(1, nghosts == 2 ? k_cfl_static<2> : k_cfl_static<4>, nblocks, 256, 0, s, U, dxdy, gamma,
+                 dt_per_cfl_out);
+  if (e == cudaSuccess) return AMR_OK;
+  cudaGetLastError();
+  return AMR_E_CUDA;
 }

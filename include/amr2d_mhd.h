@@ -310,13 +310,12 @@ int amr_adjoint_recorded(amr_handle *h, int32_t *steps);
  *                  of min(dx,dy) / max(|rho| + c_f,x, |u| + c_f,y)); NaN if a
  *                  block's wave speed is NaN (this variant has no pressure
  *                  trap)
- * The scratch (the running minimum and two counts) is in fixed file-scope
- * device variables of every GPU that loads the library; nblocks above 65536
+ * There is no scratch: the running minimum is *dt_per_cfl_out itself, and a
+ * call depends on nothing that another one left.  Calls that overlap on the
+ * GPU (different streams) need a dt_per_cfl_out each.  nblocks above 65536
  * returns AMR_E_TOO_LARGE.  The first call on a device loads the entry
  * point's kernels; make it before any stream capture, and do not use the entry
- * point after a cudaDeviceReset in the same process.
- * Calls share the variables, so calls that overlap on the GPU (different
- * streams) race: serialise them on one stream.  An error already pending in
+ * point after a cudaDeviceReset in the same process.  An error already pending in
  * the CUDA runtime is reported as AMR_E_CUDA and left for its owner.  Work
  * is enqueued on `cuda_stream`; the call does not synchronise. */
 int amr_cfl_dt_static(const double *U, int32_t nblocks, int32_t nghosts, const double *dxdy, double gamma,

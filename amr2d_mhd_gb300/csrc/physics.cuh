@@ -234,12 +234,17 @@ __device__ __forceinline__ T fast_speed(M &m, const T *w, T gamma, int norm) {
 
 // FP32 faces: the squares of the sound and Alfven speeds as they are, without
 // the roots that the FP64 path takes and squares again, and the transverse
-// field's share as a sum instead of a difference (fewer roundings, and never negative)
+// field's share as a sum instead of a difference (fewer roundings, and never
+// negative).  A negative square is NaN, as its root is there: the trap for face
+// states of negative pressure or density.
+__device__ __forceinline__ float real_speed(float a2, float c2, float cf) {
+  return fminf(a2, c2) < 0.f ? __int_as_float(0x7fffffff) : cf;
+}
 __device__ __forceinline__ float fast_speed_of(Quick &m, const float *w, float gamma) {
   const float ir = m.div(1.f, w[0]);
   const float t2 = (w[6] * w[6] + w[7] * w[7]) * ir, c2 = w[5] * w[5] * ir + t2, a2 = gamma * w[4] * ir;
   const float d = c2 - a2;
-  return m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * t2)));
+  return real_speed(a2, c2, m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * t2))));
 }
 
 // the same for norm 5 (x) and 6 (y), whose first two terms are the same values
@@ -260,8 +265,8 @@ __device__ __forceinline__ void fast_speeds_of(Native<float> &m, const float *w,
   const float ir = 1.f / w[0];
   const float bx = w[5] * w[5] * ir, by = w[6] * w[6] * ir, bz = w[7] * w[7] * ir, a2 = gamma * w[4] * ir;
   const float c2 = bx + by + bz, d = c2 - a2;
-  cf[0] = m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (by + bz))));
-  cf[1] = m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (bx + bz))));
+  cf[0] = real_speed(a2, c2, m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (by + bz)))));
+  cf[1] = real_speed(a2, c2, m.root(0.5f * (c2 + a2 + m.root(d * d + 4.f * a2 * (bx + bz)))));
 }
 template <class M>
 __device__ __forceinline__ void fast_speeds_of(M &m, const double *w, double gamma, double *cf) {

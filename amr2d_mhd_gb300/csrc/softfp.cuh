@@ -333,6 +333,7 @@ AMR_HD double times_pow2(double x, double p, bool &bad) {
 template <typename T>
 struct Native {
   __device__ __forceinline__ T div(T a, T b) { return a / b; }
+  __device__ __forceinline__ T ratio(T a, T b) { return a / b; }   // b not subnormal (Quick)
   __device__ __forceinline__ T root(T x) { return sqrt(x); }
   template <int B> __device__ __forceinline__ T by(T a) { return a / T(B); }
   __device__ __forceinline__ T mul(T a, T b) { return a * b; }
@@ -358,6 +359,7 @@ struct Native {
 struct Soft {
   bool bad = false;
   __device__ __forceinline__ double div(double a, double b) { return div_rn(a, b, bad); }
+  __device__ __forceinline__ double ratio(double a, double b) { return div(a, b); }
   __device__ __forceinline__ double root(double x) { return sqrt_rn(x, bad); }
   template <int B> __device__ __forceinline__ double by(double a) { return div_by<B>(a, bad); }
   __device__ __forceinline__ double mul(double a, double b) { return mul_rn(a, b, bad); }
@@ -380,18 +382,32 @@ struct Soft {
 // The FP32 face kernels': quotients and roots from MUFU without the
 // compiler's handling of subnormal operands (2 and 1 instructions; a quotient
 // is a * rcp(b), within 2 ulp, and quotients of one b share the reciprocal).
+// MUFU takes a divisor above 2^126 for infinite (reciprocal zero) and a
+// subnormal divisor or radicand for zero: `low`, the smallest of all three,
+// notes those, and the face is then evaluated again with Native, as after Soft.
+// (The check costs 1 % of a step of 32 MC + HLLD rotors or 24 HLLE blasts, 3.5 %
+// of a 512^2 WENO3 layer.)
 struct Quick : Native<float> {
+  float low = 1.0f;
   __device__ __forceinline__ float div(float a, float b) {
+    low = fminf(low, fabsf(b));
+    return ratio(a, b);
+  }
+  // a / b where a zero b is as good as any (infinite or NaN, as IEEE) and a subnormal one does not occur
+  __device__ __forceinline__ float ratio(float a, float b) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    low = fminf(low, fabsf(r));
     return a * r;
   }
   __device__ __forceinline__ float root(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    low = fminf(low, fabsf(x));
     return r;
   }
   template <int B> __device__ __forceinline__ float by(float a) { return a * (1.0f / B); }
+  __device__ __forceinline__ bool failed() const { return low < 0x1p-126f; }
 };
 template <typename T> struct FaceArith { using type = Soft; };
 template <> struct FaceArith<float> { using type = Quick; };

@@ -265,19 +265,6 @@ __device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, boo
   return riemann<FLUX, T>(m, wl, wr, gamma, fl);
 }
 
-// the same with the native operators, for the rare face whose operands left
-// the range of the Soft arithmetic; a function of its own, so that its
-// registers are not the hot path's.  The flux goes to its planes of `out`.
-template <int RECON, int FLUX, int NN, typename T>
-__device__ __noinline__ int face_flux_native(const T *W, int cL, int s, bool yf, int lim, T h, T bn, T gamma, T *out) {
-  Native<T> m;
-  T fl[8];
-  const int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, lim, h, bn, gamma, fl);
-#pragma unroll
-  for (int k = 0; k < 8; k++) out[face_plane(k, yf) * NN] = fl[k];
-  return rc;
-}
-
 // resident CTAs per SM the fused stage kernel is compiled for: the FP32
 // instantiation trades registers for occupancy (it is latency-bound)
 template <typename S> struct StageMinBlocks { static constexpr int value = 1; };
@@ -286,6 +273,51 @@ template <typename S> struct StageThreads { static constexpr int value = 256; };
 template <> struct StageThreads<float> { static constexpr int value = AMR_STAGE_F32_THREADS; };
 template <typename S> struct StageKeepU { static constexpr bool value = false; };
 template <> struct StageKeepU<float> { static constexpr bool value = AMR_STAGE_F32_KEEPU != 0; };
+
+// One face of the fused stage, evaluated with the arithmetic M: its flux to the
+// block's faces in shared memory and to ff / gg.  False, with nothing stored
+// or reported, if an operand left M's range.
+template <int NG, int RECON, int FLUX, typename S, class M>
+__device__ __forceinline__ bool stage_face(const StageArgs &a, const LeafTask &task, const S *sW, S *sFx, S *sFy,
+                                           int lim, S gamma, int f) {
+  using G = Geo<NG>;
+  constexpr int N = G::N, NN = G::NN, LO = G::LO, NF = G::NF, NFX = G::NFX;
+  const bool yf = f >= NF * NF;
+  const int g = yf ? f - NF * NF : f;
+  const int r = g / NF, c = g % NF;
+  // cell-index stride along the face normal and the left cell of the face
+  const int s = yf ? N : 1;
+  const int cL = (LO + r) * N + (LO + c);
+  const int fpos = cL + s;  // face index of the reference = the right cell
+  const S h = static_cast<S>(yf ? task.dy : task.dx);
+  const S bn = static_cast<S>(a.B[static_cast<size_t>(task.slot) * 2 * NN + (yf ? NN : 0) + fpos]);
+  S fl[8];
+  M m;
+  const int rc = face_flux_of<RECON, FLUX, NN, S>(m, sW, cL, s, yf, lim, h, bn, gamma, fl);
+  if (m.failed()) return false;
+  if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
+  S *out = static_cast<S *>(yf ? a.gg : a.ff) + static_cast<size_t>(task.slot) * 8 * NN + fpos;
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    bad |= bits_nan(fl[k]);
+    const int p = face_plane(k, yf);
+    if (!yf) sFx[(p * NF + r) * NFX + (c + 1)] = fl[k];
+    else sFy[(p * NFX + (r + 1)) * NF + c] = fl[k];
+    out[p * NN] = fl[k];
+  }
+  if (bad) dev_fail(a.err, DERR_NAN, task.slot, fpos % N, fpos / N, 0.0);
+  return true;
+}
+// the same with the native operators, for the rare face whose operands left
+// the range of the Soft or Quick arithmetic; a function of its own, so that its
+// registers are not the hot path's
+template <int NG, int RECON, int FLUX, typename S>
+__device__ __noinline__ void stage_face_native(const StageArgs &a, int ti, const S *sW, S *sFx, S *sFy, int f) {
+  const LeafTask task = a.tasks[ti];
+  const InstParams ip = a.inst[task.inst];
+  stage_face<NG, RECON, FLUX, S, Native<S>>(a, task, sW, sFx, sFy, ip.limiter, static_cast<S>(ip.gamma), f);
+}
 
 // One leaf block of the fused stage: task `ti`, its conserved state staged
 // into shared memory by a bulk copy completing on `bar` (initialised by the
@@ -365,38 +397,14 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   // 2. Riemann fluxes at x faces (i+1/2, j), i in [LO, HI], and y faces
   const T gamma = static_cast<T>(ip.gamma);
   const int lim = ip.limiter;
-  for (int f = tid; f < 2 * NF * NF; f += nthr) {
-    const bool yf = f >= NF * NF;
-    const int g = yf ? f - NF * NF : f;
-    const int r = g / NF, c = g % NF;
-    // cell-index stride along the face normal and the left cell of the face
-    const int s = yf ? N : 1;
-    const int cL = (LO + r) * N + (LO + c);
-    const int fpos = cL + s;  // face index of the reference = the right cell
-    const T h = static_cast<T>(yf ? task.dy : task.dx);
-    const T bn = static_cast<T>(yf ? By[fpos] : Bx[fpos]);
-    T fl[8];
-    typename FaceArith<T>::type m;
-    int rc = face_flux_of<RECON, FLUX, NN, T>(m, sW, cL, s, yf, lim, h, bn, gamma, fl);
-    if (m.failed()) {
-      T *out = (yf ? gg : ff) + fpos;
-      rc = face_flux_native<RECON, FLUX, NN, T>(sW, cL, s, yf, lim, h, bn, gamma, out);
-#pragma unroll
-      for (int k = 0; k < 8; k++) fl[k] = out[face_plane(k, yf) * NN];
-    }
-    if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
-    bool bad = false;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      bad |= bits_nan(fl[k]);
-      const int p = face_plane(k, yf);
-      if (!yf) sFx[(p * NF + r) * NFX + (c + 1)] = fl[k];
-      else sFy[(p * NFX + (r + 1)) * NF + c] = fl[k];
-      (yf ? gg : ff)[p * NN + fpos] = fl[k];
-    }
-    if (bad) dev_fail(a.err, DERR_NAN, task.slot, fpos % N, fpos / N, 0.0);
+  unsigned again = 0, round = 1;   // the rounds whose face is to be repeated (after the loop, which keeps no room for the call)
+  for (int f = tid; f < 2 * NF * NF; f += nthr, round <<= 1)
+    if (!stage_face<NG, RECON, FLUX, S, typename FaceArith<S>::type>(a, task, sW, sFx, sFy, lim, gamma, f)) again |= round;
+  if (__syncthreads_or(again)) {
+    for (int f = tid; again; f += nthr, again >>= 1)
+      if (again & 1) stage_face_native<NG, RECON, FLUX, S>(a, ti, sW, sFx, sFy, f);
+    __syncthreads();
   }
-  __syncthreads();
 
   // 3. residual on [LO, HI]^2 (zero elsewhere) and the RK stage on every cell
   const T dt = static_cast<T>(ip.dt);
@@ -441,7 +449,7 @@ __device__ __forceinline__ void stage_bar_init(uint64_t *bar) {
 // few blocks, whose 640 threads take the 578 faces in one round.
 constexpr int kStageWide = 640;
 template <int NG, int RECON, int FLUX, typename S, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinBlocks<S>::value) k_stage(StageArgs a) {
+__global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinBlocks<S>::value) k_stage(const __grid_constant__ StageArgs a) {
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   stage_bar_init(&bar);
@@ -453,7 +461,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinB
 // counter (the mbarrier phase alternates per block); the last CTA to finish
 // zeroes the counters for the next launch
 template <int NG, int RECON, int FLUX, typename S>
-__global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::value) k_stage_dyn(StageArgs a) {
+__global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::value) k_stage_dyn(const __grid_constant__ StageArgs a) {
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   __shared__ int next;

@@ -58,9 +58,12 @@ cudaError_t launch_stage_flux(const Method &m, const StageArgs &a, int ntasks, c
 // for: 4 (128 registers) for Rusanov and for WENO5, whose spills cost less
 // than the fourth CTA brings (256^2 KH, MC + RUSA: 1547 against 1581 us per
 // 4-step pass with 3; Orszag-Tang, WENO5 + HLLD: 1714 against 1821), 3 for
-// the rest (rotor, MC + HLLD: 1610 against 1655 us with 4).
-template <int RECON, int FLUX>
+// the rest (rotor, MC + HLLD: 1610 against 1655 us with 4).  FP32: 8 (64
+// registers; WENO5 6, 80), what the face itself takes; left free, the native
+// repetition would set the kernel's registers, 68 to 127.
+template <int RECON, int FLUX, typename S>
 constexpr int faces_minb() {
+  if (sizeof(S) == 4) return RECON == REC_WENO5 ? 6 : 8;
   return RECON == REC_WENO5 || FLUX == FLX_RUSA ? 4 : 3;
 }
 
@@ -92,9 +95,9 @@ cudaError_t launch_faces_t(const SplitArgs &a, int block, int persistent, int pd
     }
     if (!ps) {
       cudaError_t e = persistent == 2
-          ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_faces_dyn<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX>())>,
+          ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_faces_dyn<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX, S>())>,
                                                           block, 0)
-          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_faces_persist<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX>())>,
+          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, k_faces_persist<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX, S>())>,
                                                           block, 0);
       if (e != cudaSuccess) return e;
       if (ps < 1) ps = 1;
@@ -102,12 +105,12 @@ cudaError_t launch_faces_t(const SplitArgs &a, int block, int persistent, int pd
     const size_t cap = static_cast<size_t>(sms) * ps;
     if (grid > cap) grid = cap;
     if (persistent == 2)
-      return launch_k(pdl, k_faces_dyn<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX>())>, static_cast<unsigned>(grid), block, 0,
+      return launch_k(pdl, k_faces_dyn<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX, S>())>, static_cast<unsigned>(grid), block, 0,
                       s, a);
-    return launch_k(pdl, k_faces_persist<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX>())>, static_cast<unsigned>(grid), block, 0,
+    return launch_k(pdl, k_faces_persist<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX, S>())>, static_cast<unsigned>(grid), block, 0,
                     s, a);
   }
-  return launch_k(pdl, k_faces<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX>())>, static_cast<unsigned>(grid), block, 0, s, a);
+  return launch_k(pdl, k_faces<NG, RECON, FLUX, S, (faces_minb<RECON, FLUX, S>())>, static_cast<unsigned>(grid), block, 0, s, a);
 }
 
 template <int FLUX, typename S>

@@ -91,8 +91,10 @@ __global__ void __launch_bounds__(512) k_prim_task(SplitArgs a) {
 // are bound by the FP64 pipe (76-80 % busy with 12 warps per SM): about 230
 // FP64 instructions per MC + RUSA face and 330 per MC + HLLD face, all of them
 // additions and multiplications (softfp.cuh takes the rest).
-template <int NG, int RECON, int FLUX, typename S>
-__device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
+// False, with nothing stored or reported, if an operand left the range of the
+// arithmetic M.
+template <int NG, int RECON, int FLUX, typename S, class M>
+__device__ __forceinline__ bool face_flux_with(const SplitArgs &a, size_t e) {
   using G = Geo<NG>;
   using T = S;
   constexpr int N = G::N, NN = G::NN, LO = G::LO, NF = G::NF, PER = 2 * NF * NF;
@@ -112,13 +114,9 @@ __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
   const T bn = static_cast<T>(Bf[fpos]);
   S *out = static_cast<S *>(yf ? a.gg : a.ff) + base + fpos;
   T fl[8];
-  typename FaceArith<T>::type m;
-  int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, ip.limiter, h, bn, gamma, fl);
-  if (m.failed()) {
-    rc = face_flux_native<RECON, FLUX, NN, T>(W, cL, s, yf, ip.limiter, h, bn, gamma, out);
-#pragma unroll
-    for (int k = 0; k < 8; k++) fl[k] = out[face_plane(k, yf) * NN];
-  }
+  M m;
+  const int rc = face_flux_of<RECON, FLUX, NN, T>(m, W, cL, s, yf, ip.limiter, h, bn, gamma, fl);
+  if (m.failed()) return false;
   if (rc) dev_fail(a.err, rc, task.slot, fpos % N, fpos / N, 0.0);
   bool bad = false;
 #pragma unroll
@@ -127,10 +125,23 @@ __device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
     out[face_plane(k, yf) * NN] = fl[k];
   }
   if (bad) dev_fail(a.err, DERR_NAN, task.slot, fpos % N, fpos / N, 0.0);
+  return true;
+}
+
+// the same with the native operators, for the rare face whose operands left
+// the range of the Soft or Quick arithmetic; a function of its own, so that its
+// registers are not the hot path's
+template <int NG, int RECON, int FLUX, typename S>
+__device__ __noinline__ void face_flux_native(const SplitArgs &a, size_t e) {
+  face_flux_with<NG, RECON, FLUX, S, Native<S>>(a, e);
+}
+template <int NG, int RECON, int FLUX, typename S>
+__device__ __forceinline__ void face_flux(const SplitArgs &a, size_t e) {
+  if (!face_flux_with<NG, RECON, FLUX, S, typename FaceArith<S>::type>(a, e)) face_flux_native<NG, RECON, FLUX, S>(a, e);
 }
 
 template <int NG, int RECON, int FLUX, typename S, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_faces(SplitArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_faces(const __grid_constant__ SplitArgs a) {
   pdl_wait();
   constexpr int PER = 2 * Geo<NG>::NF * Geo<NG>::NF;
   const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -141,7 +152,7 @@ __global__ void __launch_bounds__(128, MINB) k_faces(SplitArgs a) {
 // persistent variant: a grid sized to the CTAs the SMs hold at once walks
 // the whole face list of the step (all leaf blocks of all instances)
 template <int NG, int RECON, int FLUX, typename S, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_faces_persist(SplitArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_faces_persist(const __grid_constant__ SplitArgs a) {
   pdl_wait();
   constexpr int PER = 2 * Geo<NG>::NF * Geo<NG>::NF;
   const size_t n = static_cast<size_t>(a.ntasks) * PER;
@@ -157,7 +168,7 @@ __global__ void __launch_bounds__(128, MINB) k_faces_persist(SplitArgs a) {
 // CTA to finish zeroes the counters for the next launch (every CTA has left
 // its loop by then, so nothing claims work any more)
 template <int NG, int RECON, int FLUX, typename S, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_faces_dyn(SplitArgs a) {
+__global__ void __launch_bounds__(128, MINB) k_faces_dyn(const __grid_constant__ SplitArgs a) {
   pdl_wait();
   constexpr int PER = 2 * Geo<NG>::NF * Geo<NG>::NF;
   const unsigned n = static_cast<unsigned>(a.ntasks) * PER;

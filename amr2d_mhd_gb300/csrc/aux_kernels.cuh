@@ -182,12 +182,12 @@ __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f
     // products and halvings on the integer pipe: as FP64 instructions they
     // were most of the pipe's work, which bound this kernel in batches (6272
     // FP32 leaves, predictor and corrector: 58 and 84 us before, 50 and 51 now)
-    const double e0 = E[c], ey = E[jp * N + i] - e0, ex = e0 - E[j * N + ip];   // ex: minus the reference's
+    const double e0 = E[c], ey = E[jp * N + i] - e0, ex = E[j * N + ip] - e0;
     double bx = B0[c], by = B0[NN + c], nx = 0, ny = 0;
     if (a.step != 1) { bx += B1[c]; by += B1[NN + c]; }
     evaluate<double>([&](auto &m) {
       nx = m.scaled(bx - m.mul(dt, m.mul(t.rcp_dy, ey)), part);
-      ny = m.scaled(by - m.mul(dt, m.mul(t.rcp_dx, ex)), part);
+      ny = m.scaled(by - m.mul(dt, m.mul(-t.rcp_dx, ex)), part);
     });
     B1[c] = nx;
     B1[NN + c] = ny;

@@ -128,7 +128,7 @@ int Engine::ct2d_taped(int step) {
   a.Bsrc = step == 1 ? Bi_ : Bis_;
   a.Bnew = step == 1 ? Bis_ : Bi_;
   a.q = step == 1 ? Us_ : U_;
-  a.err = h_err_.as<DevError>();
+  a.err = d_err_.as<DevError>();
   a.step = step;
   const int n = static_cast<int>(tasks_.size());
   const size_t cell = sizeof(double) * 8 * nn_ * used_slots_, face = sizeof(double) * 2 * nn_ * used_slots_;

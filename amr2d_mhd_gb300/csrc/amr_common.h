@@ -16,7 +16,7 @@ enum Recon { REC_MUSCL = 0, REC_WENO3 = 1, REC_WENO5 = 2 };
 // Riemann solvers (riemannS.cpp:30-44)
 enum Flux { FLX_RUSA = 0, FLX_HLLE, FLX_HLLC, FLX_HLLD, FLX_ROE };
 
-// device error word: first failure wins (code, block, i, j)
+// device error record: first failure wins (code, block, i, j)
 enum DevErr { DERR_NONE = 0, DERR_PRESSURE = 1, DERR_NAN = 2, DERR_HLLC = 3, DERR_REFINE_NAN = 4, DERR_TIMEOUT = 5,
               DERR_PSI = 6 };
 struct DevError {
@@ -24,6 +24,7 @@ struct DevError {
   int blk;
   int i, j;
   double value;
+  DevError *host;   // of the record in device memory: the page-locked one that the host reads
 };
 
 // One leaf block to process: its physical slot and the instance it belongs to.

@@ -79,7 +79,7 @@ Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
   for (void *p : {U_, Us_, ff_, gg_, W_}) if (p) cudaFree(p);
   for (double *p : {Bi_, Bis_, EMF_}) if (p) cudaFree(p);
-  for (DevBuf *b : {&d_tasks_, &d_params_, &d_grad_, &d_snap_, &d_treeops_, &d_stage_,
+  for (DevBuf *b : {&d_tasks_, &d_params_, &d_grad_, &d_err_, &d_snap_, &d_treeops_, &d_stage_,
                     &d_ctr_, &d_snap3_, &d_bar_})
     b->release();
   d_ops_.release();
@@ -203,7 +203,9 @@ int Engine::create(const amr_config *cfgs, int n) {
   CK(d_bar_.ensure(2 * sizeof(unsigned)), "alloc");   // k_ct_coop's grid barrier (count, generation)
   CK(cudaMemsetAsync(d_bar_.p, 0, 2 * sizeof(unsigned), stream_), "memset");
   CK(h_err_.ensure(sizeof(DevError)), "alloc");
-  std::memset(h_err_.p, 0, sizeof(DevError));
+  CK(d_err_.ensure(sizeof(DevError)), "alloc");
+  *h_err_.as<DevError>() = DevError{0, 0, 0, 0, 0.0, h_err_.as<DevError>()};
+  CK(cudaMemcpyAsync(d_err_.p, h_err_.p, sizeof(DevError), cudaMemcpyHostToDevice, stream_), "h2d");
   CK(h_params_.ensure(sizeof(InstParams) * n), "alloc");
   CK(d_params_.ensure(sizeof(InstParams) * n), "alloc");
   return AMR_OK;
@@ -633,7 +635,7 @@ int Engine::stage(int step, const FillFuse *fuse) {
     a.B = step == 1 ? Bi_ : Bis_;
     a.ff = ff_;
     a.gg = gg_;
-    a.err = h_err_.as<DevError>();
+    a.err = d_err_.as<DevError>();
     a.ctr = d_ctr_.as<unsigned>();
     a.step = step;
     a.ntasks = n;
@@ -653,7 +655,7 @@ int Engine::stage(int step, const FillFuse *fuse) {
     a.B = step == 1 ? Bi_ : Bis_;
     a.ff = ff_;
     a.gg = gg_;
-    a.err = h_err_.as<DevError>();
+    a.err = d_err_.as<DevError>();
     a.ctr = d_ctr_.as<unsigned>();
     a.step = step;
     a.ntasks = n;
@@ -774,7 +776,7 @@ int Engine::ct2d(int step, const FillPass *in, const FillPass *out, int emf_buf,
   a.Bsrc = step == 1 ? Bi_ : Bis_;
   a.Bnew = step == 1 ? Bis_ : Bi_;
   a.q = step == 1 ? Us_ : U_;
-  a.err = h_err_.as<DevError>();
+  a.err = d_err_.as<DevError>();
   a.step = step;
   const int n = static_cast<int>(tasks_.size());
   a.ntasks = n;
@@ -814,7 +816,7 @@ int Engine::dt_crit(bool want_grad, const FillFuse *fuse) {
   a.U = U_;
   a.lambda = h_lambda_.as<double>();
   a.grad = h_grad_.as<double>();
-  a.err = h_err_.as<DevError>();
+  a.err = d_err_.as<DevError>();
   a.want_grad = want_grad ? 1 : 0;
   if (fuse) a.fuse = *fuse;
   CK(launch_dt_cell(m_, a, static_cast<int>(tasks_.size()), stream_), "dt kernel");

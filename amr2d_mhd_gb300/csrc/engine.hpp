@@ -198,7 +198,7 @@ class Engine {
   int64_t nops_ = 0, nsnaps_ = 0, hole_ops_ = 0;
   int compile_programs();          // recompile changed instances (host threads)
   int layout_programs(bool relayout);
-  DevBuf d_tasks_, d_params_, d_grad_, d_snap_, d_ops_, d_snaps_;
+  DevBuf d_tasks_, d_params_, d_grad_, d_err_, d_snap_, d_ops_, d_snaps_;
   DevBuf d_treeops_, d_stage_, d_ctr_;
   DevBuf d_snap3_;                 // fused fills: three rotating snapshot buffers
   DevBuf d_bar_;                   // grid barrier of the cooperative CT launch

@@ -147,7 +147,7 @@ int Engine::admesh_all(const std::vector<int> &which, const std::vector<std::vec
   a.inst = d_params_.as<InstParams>();
   a.U = U_;
   a.Bi = Bi_;
-  a.err = h_err_.as<DevError>();
+  a.err = d_err_.as<DevError>();
   CK(launch_refine(m_, a, static_cast<int>(ref.size()), stream_), "refine");
   a.ops = d_treeops_.as<TreeOp>() + ref.size();
   CK(launch_coarsen(m_, a, static_cast<int>(crs.size()), stream_), "coarsen");

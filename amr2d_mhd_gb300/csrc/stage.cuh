@@ -48,12 +48,18 @@ struct StageArgs {
 // small kernels.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The first failure is claimed in device memory and written to the record that
+// the host reads after the step.  (A state that fails in every cell and face
+// makes millions of claims: a step of 4096 blocks with 9.7 M of them takes 14 ms,
+// 112 with the claims in host memory.)
 __device__ __forceinline__ void dev_fail(DevError *e, int code, int blk, int i, int j, double v) {
   if (atomicCAS(&e->code, 0, code) == 0) {
-    e->blk = blk;
-    e->i = i;
-    e->j = j;
-    e->value = v;
+    DevError *h = e->host;
+    h->code = code;
+    h->blk = blk;
+    h->i = i;
+    h->j = j;
+    h->value = v;
   }
 }
 

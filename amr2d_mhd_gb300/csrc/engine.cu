@@ -692,10 +692,10 @@ int Engine::autotune(int reps, char *report, size_t len) {
   struct Cand { bool split; int fb, cb, gb, pers; float ms; };
   std::vector<Cand> cands;
   for (int gb : {128, 256, 512}) {
-    cands.push_back({false, 128, 256, gb, 0, 0.f});
-    cands.push_back({false, 128, 256, gb, 2, 0.f});   // fused, persistent over the leaf list
+    cands.push_back({false, 0, 256, gb, 0, 0.f});
+    cands.push_back({false, 0, 256, gb, 2, 0.f});   // fused, persistent over the leaf list
     for (int pers : {0, 1, 2})
-      for (int fb : {64, 128})
+      for (int fb : {pers == 0 ? 32 : 64, 128})
         for (int cb : {256, 512}) cands.push_back({true, fb, cb, gb, pers, 0.f});
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -750,9 +750,12 @@ int Engine::autotune(int reps, char *report, size_t len) {
     std::string s;
     char line[160];
     for (const Cand &c : cands) {
-      std::snprintf(line, sizeof line, "%s%s faces %d%s cells %d ghosts %d: %.4f ms\n", &c == best ? "* " : "  ",
-                    c.split ? "split" : "fused", c.fb, c.pers == 2 ? " dynamic" : (c.pers ? " persistent" : ""), c.cb,
-                    c.gb, c.ms);  // fused + dynamic: k_stage_dyn
+      const char *how = c.pers == 2 ? " dynamic" : (c.pers ? " persistent" : "");   // fused + dynamic: k_stage_dyn
+      if (c.split)
+        std::snprintf(line, sizeof line, "%ssplit faces %d%s cells %d ghosts %d: %.4f ms\n", &c == best ? "* " : "  ",
+                      c.fb, how, c.cb, c.gb, c.ms);
+      else
+        std::snprintf(line, sizeof line, "%sfused%s ghosts %d: %.4f ms\n", &c == best ? "* " : "  ", how, c.gb, c.ms);
       s += line;
     }
     std::strncpy(report, s.c_str(), len - 1);

@@ -20,8 +20,9 @@ struct Method {
   int flux;    // Flux
   int f32;     // FP32 bulk storage / arithmetic
   // launch schedule (picked by Engine::autotune): threads per CTA of the
-  // face-flux kernel (64 or 128), of the per-cell kernels and of the ghost fills
-  int faces_block = 128;
+  // face-flux kernel (one-shot 32 or 128, persistent 64 or 128; else the first
+  // and the last), of the per-cell kernels and of the ghost fills
+  int faces_block = 0;
   int cell_block = 256;
   int ghost_block = 256;
   int persistent = 0;   // face fluxes by a grid of resident CTAs looping over the face list: 1 in

@@ -9,10 +9,10 @@
 namespace amr {
 
 // persistent = 2 (and a.ctr set): k_stage_dyn on a grid of the CTAs the SMs
-// hold at once; otherwise one CTA per leaf block.  Up to two FP32 blocks per SM
-// take the wide CTA in either case: with so few the launch lasts as long as
-// one block, whose rounds of faces and cells it halves (196 blocks: 18 and 16 us
-// against 26 and 24).
+// hold at once; otherwise one CTA per leaf block, the wide one for up to two FP32
+// blocks per SM: with so few the launch lasts as long as one block, whose
+// rounds of faces and cells it halves (196 blocks: 18 and 16 us against 26 and
+// 24).
 template <int NG, int RECON, int FLUX, typename S>
 cudaError_t launch_stage_t(const StageArgs &a, int ntasks, int pdl, int persistent, cudaStream_t s) {
   constexpr int smem = stage_smem_bytes<NG, S>();
@@ -35,11 +35,11 @@ cudaError_t launch_stage_t(const StageArgs &a, int ntasks, int pdl, int persiste
     attr_set = true;
   }
   if (ntasks <= 0) return cudaSuccess;
-  if (wide != threads && ntasks <= 2 * sms) return launch_k(pdl, once_wide, ntasks, wide, smem, s, a);
   if (persistent == 2 && a.ctr) {
     const int grid = ntasks < sms * per_sm ? ntasks : sms * per_sm;
     return launch_k(pdl, dyn, grid, threads, smem, s, a);
   }
+  if (wide != threads && ntasks <= 2 * sms) return launch_k(pdl, once_wide, ntasks, wide, smem, s, a);
   return launch_k(pdl, once, ntasks, threads, smem, s, a);
 }
 
@@ -67,7 +67,7 @@ constexpr int faces_minb() {
   return RECON == REC_WENO5 || FLUX == FLX_RUSA ? 4 : 3;
 }
 
-// persistent: 0 one CTA per 32 faces; 1 a grid of resident CTAs
+// persistent: 0 one CTA per `block` faces; 1 a grid of resident CTAs
 // striding over the face list; 2 the same with dynamic claims of 32 faces
 // per warp (k_faces_dyn, needs a.ctr)
 template <int NG, int RECON, int FLUX, typename S>
@@ -75,12 +75,13 @@ cudaError_t launch_faces_t(const SplitArgs &a, int block, int persistent, int pd
   constexpr int PER = 2 * Geo<NG>::NF * Geo<NG>::NF;
   const size_t n = static_cast<size_t>(a.ntasks) * PER;
   if (n == 0) return cudaSuccess;
-  if (block != 64) block = 128;  // the kernel is bounded at 128 threads per CTA
-  // The one-shot kernel takes CTAs of one warp (its warps share nothing), which
-  // spread evenly and leave no SM waiting for a CTA's last warp: rotor of 28 /
-  // 196 leaves (HLLD) 32.4 / 107 us against 34.4 / 109 with 128 threads, 88 leaves
-  // of Brio-Wu (HLLE) 46.8 against 50.7, the same for Rusanov and WENO5.
-  if (!persistent) block = 32;
+  // The one-shot kernel takes CTAs of one warp (its warps share nothing) unless
+  // asked for 128 threads: they spread evenly and leave no SM waiting for a CTA's
+  // last warp (rotor of 28 / 196 leaves, HLLD, 32.4 / 107 us against 34.4 / 109, 88
+  // leaves of Brio-Wu, HLLE, 46.8 against 50.7, the same for Rusanov and WENO5).
+  // The kernels are bounded at 128 threads per CTA.
+  if (persistent) block = block == 64 ? 64 : 128;
+  else block = block == 128 ? 128 : 32;
   size_t grid = (n + block - 1) / block;
   if (persistent == 2 && !a.ctr) persistent = 1;
   if (persistent) {

@@ -122,16 +122,17 @@ __device__ __forceinline__ void sum_sq3(float a, float b, float c, float &hi, fl
 
 // FP32 path: the pressure from the total energy, (gamma - 1) (E - (|m|^2/rho +
 // |B|^2)/2), whose cancellation is where FP32 loses digits, evaluated with
-// pairs of floats: the sums of squares (sum_sq3), |m|^2/rho with 1/rho = ir +
-// rl (rl from the FMA residual 1 - rho*ir), the sum of both halves and the
-// subtraction (TwoSum), and the product with gamma - 1 (a pair as well).
-// Every step is good to 2^-45 of the subtracted terms, which an evaluation
-// with FP64 sums does not improve on (the pairs it starts from carry that
-// error), and none is on the FP64 pipe, 12 instructions of which per cell kept
-// the FP32 path's dt kernel 76 % bound (16 clocks per warp each).  The
-// velocities are the FP32 momenta times the FP32 reciprocal.  (A component
-// above ~1.8e19 overflows its FP32 square; such a state is out of the FP32
-// path's range in any case.)
+// unevaluated sums of floats: the sums of squares (sum_sq3) and |m|^2/rho with
+// 1/rho = ir + rl (rl from the FMA residual 1 - rho*ir) as pairs, good to 2^-47 of
+// their value; their sum and the subtraction without further error (TwoSum, also
+// of the low parts, whose rounding would add half as much again); and the
+// product with gamma - 1 (a pair as well).  The error is that of the same pairs
+// summed in FP64 (rms 0.17-0.39 2^-48 of the subtracted terms, results within
+// 0.5 ulp where they do not cancel), but no instruction is on the FP64 pipe,
+// 12 of which per cell kept the FP32 path's dt kernel 76 % bound (16 clocks per
+// warp each).  The velocities are the FP32 momenta times the FP32 reciprocal.
+// (A component above ~1.8e19 overflows its FP32 square; such a state is out of
+// the FP32 path's range in any case.)
 template <>
 __device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, const GasGamma<float> &gam) {
   const float ir = 1.0f / u[0];
@@ -141,13 +142,16 @@ __device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, 
   sum_sq3(u[5], u[6], u[7], bh, bl);
   const float kh = __fmul_rn(mh, ir);
   const float kl = __fadd_rn(__fmaf_rn(mh, ir, -kh), __fadd_rn(__fmul_rn(mh, rl), __fmul_rn(ml, ir)));
-  float sh, sl, dh, dl;
+  // |m|^2/rho + |B|^2 = sh + s2 + e1 + e2, E - half of it = th + tl
+  float sh, sl, s1, e1, s2, e2, dh, dl, th, tl;
   two_sum(kh, bh, sh, sl);
-  sl = __fadd_rn(sl, __fadd_rn(kl, bl));
+  two_sum(kl, bl, s1, e1);
+  two_sum(sl, s1, s2, e2);
   two_sum(u[4], __fmul_rn(-0.5f, sh), dh, dl);
-  dl = __fmaf_rn(-0.5f, sl, dl);
-  const float ph = __fmul_rn(gam.hi, dh);
-  float p = __fadd_rn(ph, __fadd_rn(__fmaf_rn(gam.hi, dh, -ph), __fmaf_rn(gam.hi, dl, __fmul_rn(gam.lo, dh))));
+  two_sum(dh, __fmaf_rn(-0.5f, s2, dl), th, tl);
+  tl = __fmaf_rn(-0.5f, __fadd_rn(e1, e2), tl);
+  const float ph = __fmul_rn(gam.hi, th);
+  float p = __fadd_rn(ph, __fadd_rn(__fmaf_rn(gam.hi, th, -ph), __fmaf_rn(gam.hi, tl, __fmul_rn(gam.lo, th))));
   // positivity fix of the FP32 path: the FP32 conserved state can put the
   // recovered pressure below zero where the FP64 path stays positive
   if (!(p > kPressureFloor)) p = kPressureFloor;

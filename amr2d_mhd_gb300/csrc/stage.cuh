@@ -181,13 +181,6 @@ __device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, 
 #ifndef AMR_STAGE_F32_THREADS
 #define AMR_STAGE_F32_THREADS 320
 #endif
-// 1: the FP32 fused stage keeps the block's conserved state in shared memory
-// beside the primitive state, so the RK update does not read it again (no
-// gain measured: 5.60 against 5.52 ms per step of the 64-rotor batch)
-#ifndef AMR_STAGE_F32_KEEPU
-#define AMR_STAGE_F32_KEEPU 0
-#endif
-
 // ------------------------------------------------------------ bulk staging
 // One thread issues a bulk copy (TMA, cp.async.bulk) of `bytes` contiguous
 // bytes from global to shared memory, completing on an mbarrier; every
@@ -294,8 +287,6 @@ template <typename S> struct StageMinBlocks { static constexpr int value = 1; };
 template <> struct StageMinBlocks<float> { static constexpr int value = AMR_STAGE_F32_MINB; };
 template <typename S> struct StageThreads { static constexpr int value = 256; };
 template <> struct StageThreads<float> { static constexpr int value = AMR_STAGE_F32_THREADS; };
-template <typename S> struct StageKeepU { static constexpr bool value = false; };
-template <> struct StageKeepU<float> { static constexpr bool value = AMR_STAGE_F32_KEEPU != 0; };
 
 // variable 0 of face f of the block in shared memory
 template <int NG, typename S>
@@ -365,8 +356,7 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   T *sW = reinterpret_cast<T *>(smem_raw);   // [8][NN]
   T *sFx = sW + 8 * NN;                      // [8][NF][NFX]   face i = LO + col, row j = LO + r
   T *sFy = sFx + 8 * NF * NFX;               // [8][NFX][NF]   face j = LO + row, col i = LO + c
-  constexpr bool KEEPU = StageKeepU<S>::value;
-  S *sU = KEEPU ? sFy + 8 * NFX * NF : sW;   // [8][NN] the conserved state (KEEPU), else staged in sW
+  S *sU = sW;   // [8][NN] the conserved state, staged where the primitive state replaces it
 
   const LeafTask task = a.tasks[ti];
   const InstParams ip = a.inst[task.inst];
@@ -462,7 +452,7 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
         else evaluate<T>([&](auto &m) { res = m.div(gx, dx) + m.div(gy, dy); });
       }
       const int e = k * NN + c;
-      const T q = KEEPU ? sU[e] : Q[e];
+      const T q = Q[e];
       if (a.step == 1) out[e] = q - dt * res;                         // Us = U - dt res
       else out[e] = T(0.5) * (out[e] + q - dt * res);                 // U = (U + Us - dt res)/2
     }
@@ -522,7 +512,7 @@ __global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::val
 template <int NG, typename S>
 constexpr int stage_smem_bytes() {
   using G = Geo<NG>;
-  return static_cast<int>(sizeof(S)) * ((StageKeepU<S>::value ? 16 : 8) * G::NN + 2 * 8 * G::NF * G::NFX);
+  return static_cast<int>(sizeof(S)) * (8 * G::NN + 2 * 8 * G::NF * G::NFX);
 }
 
 }  // namespace amr

@@ -187,7 +187,7 @@ __device__ __forceinline__ void ct_face_block(const CtArgs &a, const FillFuse &f
     if (a.step != 1) { bx += B1[c]; by += B1[NN + c]; }
     evaluate<double>([&](auto &m) {
       nx = m.scaled(bx - m.mul(dt, m.mul(t.rcp_dy, ey)), part);
-      ny = m.scaled(by - m.mul(dt, m.mul(-t.rcp_dx, ex)), part);
+      ny = m.scaled(by + m.mul(dt, m.mul(t.rcp_dx, ex)), part);   // the reference's by - dt * (-(1/dx) * ex), same bits
     });
     B1[c] = nx;
     B1[NN + c] = ny;

@@ -165,22 +165,6 @@ __device__ __forceinline__ void cons2prim_cell<float>(const float *u, float *w, 
   w[7] = u[7];
 }
 
-// FP32 fused stage: 320 threads per CTA (the 2 x 17 x 17 = 578 faces of a
-// block in two rounds), compiled for 4 resident CTAs per SM (48 registers, 56 B
-// of spills).  It issues in 48 % of its cycles and waits on latency between its
-// phases, so residents pay.  One GB300, us per pass of 32 rotors (12 steps), 24
-// blasts (10 steps) and a 512^2 KH layer (8 steps), state transfers included:
-//   320 threads x 4 CTAs  19812  8127  2233      320 x 3  20696  8442  2404
-//   256 x 5               19776  8133  2286      192 x 6  19763  8172  2403
-//   160 x 6               19986  8275  2417      128 x 7  20600  8487  2527
-// The kernel itself on the 6272 blocks of the rotors: 460 us at first, 377 in
-// the face frame, 287 with Quick arithmetic and the pair recovery (3 CTAs).
-#ifndef AMR_STAGE_F32_MINB
-#define AMR_STAGE_F32_MINB 4
-#endif
-#ifndef AMR_STAGE_F32_THREADS
-#define AMR_STAGE_F32_THREADS 320
-#endif
 // ------------------------------------------------------------ bulk staging
 // One thread issues a bulk copy (TMA, cp.async.bulk) of `bytes` contiguous
 // bytes from global to shared memory, completing on an mbarrier; every
@@ -281,12 +265,19 @@ __device__ __forceinline__ int face_flux_of(M &m, const T *W, int cL, int s, boo
   return riemann<FLUX, T>(m, wl, wr, gamma, fl);
 }
 
-// resident CTAs per SM the fused stage kernel is compiled for: the FP32
-// instantiation trades registers for occupancy (it is latency-bound)
-template <typename S> struct StageMinBlocks { static constexpr int value = 1; };
-template <> struct StageMinBlocks<float> { static constexpr int value = AMR_STAGE_F32_MINB; };
-template <typename S> struct StageThreads { static constexpr int value = 256; };
-template <> struct StageThreads<float> { static constexpr int value = AMR_STAGE_F32_THREADS; };
+// Threads of the fused stage's CTA and resident CTAs per SM it is compiled for.
+// FP32: 256 and 5 (48 registers), with four ghost layers 320 and 4.  The kernel
+// issues in half of its cycles and waits on latency between its phases, so
+// residents pay, up to the registers.  One GB300, us per pass of 32 rotors (12
+// steps), 24 blasts (10 steps) and a 512^2 KH layer (8 steps), state transfers
+// included:
+//   256 threads x 5 CTAs  16342  6598  1768      320 x 4  16737  6730  1794
+//   192 x 6               16448  6713  1831      320 x 3  17460  6966  1855
+// and per step of a WENO5 + HLLD layer of 18 x 18 / 21 x 21 / 25 x 25 / 40 x 40
+// blocks: 256 x 5 112 / 117 / 154 / 340, 320 x 4 108 / 113 / 157 / 336.
+template <int NG, typename S> struct StageShape { static constexpr int threads = 256, min_blocks = 1; };
+template <> struct StageShape<2, float> { static constexpr int threads = 256, min_blocks = 5; };
+template <> struct StageShape<4, float> { static constexpr int threads = 320, min_blocks = 4; };
 
 // variable 0 of face f of the block in shared memory
 template <int NG, typename S>
@@ -332,14 +323,18 @@ __device__ __forceinline__ bool stage_face(const StageArgs &a, const LeafTask &t
   return true;
 }
 // the same with the native operators, for the rare face whose operands left
-// the range of the Soft or Quick arithmetic (inline, with its arguments read
-// again: as a function of its own it costs FP32 batches 1 %, in registers kept
-// for the call)
+// the range of the Soft or Quick arithmetic, with its arguments read again.
+// FP64 calls it as a function of its own from the loop over the faces; FP32 has
+// it inline after the loop, as the registers kept for a call cost batches 1 %.
 template <int NG, int RECON, int FLUX, typename S>
 __device__ __forceinline__ void stage_face_native(const StageArgs &a, int ti, const S *sW, S *sFx, S *sFy, int f) {
   const LeafTask task = a.tasks[ti];
   const InstParams ip = a.inst[task.inst];
   stage_face<NG, RECON, FLUX, S, Native<S>>(a, task, sW, sFx, sFy, ip.limiter, static_cast<S>(ip.gamma), f);
+}
+template <int NG, int RECON, int FLUX, typename S>
+__device__ __noinline__ void stage_face_call(const StageArgs &a, int ti, const S *sW, S *sFx, S *sFy, int f) {
+  stage_face_native<NG, RECON, FLUX, S>(a, ti, sW, sFx, sFy, f);
 }
 
 // One leaf block of the fused stage: task `ti`, its conserved state staged
@@ -419,14 +414,20 @@ __device__ __forceinline__ bool stage_block(const StageArgs &a, int ti, uint64_t
   // 2. Riemann fluxes at x faces (i+1/2, j), i in [LO, HI], and y faces
   const T gamma = static_cast<T>(ip.gamma);
   const int lim = ip.limiter;
-  // faces to be repeated are marked by a NaN and taken after the loop
+  // FP32 faces to be repeated are marked by a NaN and taken after the loop
   bool again = false;
   for (int f = tid; f < 2 * NF * NF; f += nthr)
     if (!stage_face<NG, RECON, FLUX, S, typename FaceArith<S>::type>(a, task, sW, sFx, sFy, lim, gamma, f)) {
-      again = true;
-      *face_slot<NG>(sFx, sFy, f) = T(NAN);
+      if (sizeof(S) == 8) {
+        stage_face_call<NG, RECON, FLUX, S>(a, ti, sW, sFx, sFy, f);
+      } else {
+        again = true;
+        *face_slot<NG>(sFx, sFy, f) = T(NAN);
+      }
     }
-  if (__syncthreads_or(again)) {
+  if (sizeof(S) == 8) {
+    __syncthreads();
+  } else if (__syncthreads_or(again)) {
     for (int f = tid; f < 2 * NF * NF; f += nthr)
       if (bits_nan(*face_slot<NG>(sFx, sFy, f))) stage_face_native<NG, RECON, FLUX, S>(a, ti, sW, sFx, sFy, f);
     __syncthreads();
@@ -471,11 +472,11 @@ __device__ __forceinline__ void stage_bar_init(uint64_t *bar) {
   __syncthreads();
 }
 
-// One CTA per leaf block.  THREADS: StageThreads, or kStageWide for FP32 and
+// One CTA per leaf block.  THREADS: StageShape's, or kStageWide for FP32 and
 // few blocks, whose 640 threads take the 578 faces in one round.
 constexpr int kStageWide = 640;
 template <int NG, int RECON, int FLUX, typename S, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinBlocks<S>::value) k_stage(const __grid_constant__ StageArgs a) {
+__global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageShape<NG, S>::min_blocks) k_stage(const __grid_constant__ StageArgs a) {
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   stage_bar_init(&bar);
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kStageWide ? 2 : StageMinB
 // counter (the mbarrier phase alternates per block); the last CTA to finish
 // zeroes the counters for the next launch
 template <int NG, int RECON, int FLUX, typename S>
-__global__ void __launch_bounds__(StageThreads<S>::value, StageMinBlocks<S>::value) k_stage_dyn(const __grid_constant__ StageArgs a) {
+__global__ void __launch_bounds__(StageShape<NG, S>::threads, StageShape<NG, S>::min_blocks) k_stage_dyn(const __grid_constant__ StageArgs a) {
   pdl_wait();
   __shared__ __align__(8) uint64_t bar;
   __shared__ int next;

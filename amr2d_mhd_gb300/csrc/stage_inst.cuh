@@ -16,7 +16,7 @@ namespace amr {
 template <int NG, int RECON, int FLUX, typename S>
 cudaError_t launch_stage_t(const StageArgs &a, int ntasks, int pdl, int persistent, cudaStream_t s) {
   constexpr int smem = stage_smem_bytes<NG, S>();
-  constexpr int threads = StageThreads<S>::value, wide = sizeof(S) == 4 ? kStageWide : threads;
+  constexpr int threads = StageShape<NG, S>::threads, wide = sizeof(S) == 4 ? kStageWide : threads;
   auto once = k_stage<NG, RECON, FLUX, S, threads>;
   auto once_wide = k_stage<NG, RECON, FLUX, S, wide>;
   auto dyn = k_stage_dyn<NG, RECON, FLUX, S>;

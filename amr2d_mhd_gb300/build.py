@@ -1,16 +1,18 @@
 """Build of the sm_103a library libamr2d_mhd.so and of the host program
 amr2d_mhd that drives it (in-tree, amr2d_mhd_gb300/_build/).
 
-Every translation unit compiles in parallel with nvcc for sm_103a only.  Every
-translation unit but the FP32 stage and face kernels (stage_f32_*.cu,
-faces_f32_*.cu) is compiled with
--fmad=false and the host code with -ffp-contract=off: that path reproduces the reference's
-floating-point operations one by one, so nothing may be fused.  The FP32 stage
-kernels (the FP32 bulk path's reconstruction, Riemann fluxes and RK update)
-use FMA contraction and the approximate FP32 division and square root
-(-prec-div=false -prec-sqrt=false, about 2 ulp): their results are compared
-with the FP64 path through a tolerance, and the FP64 parts of that path
-(pressure recovery, face field, dt) are compiled elsewhere or stay FP64.
+Every translation unit compiles in parallel with nvcc for sm_103a only.  All but
+the FP32 stage and face kernels (stage_f32_*.cu, faces_f32_*.cu) and the adjoint
+are compiled with -fmad=false, and the host code with -ffp-contract=off: the
+FP64 path reproduces the reference's floating-point operations one by one, so
+nothing may be fused.  The FP32 stage and face kernels (reconstruction, Riemann
+fluxes and RK update of the FP32 bulk path) use FMA contraction and the
+approximate FP32 division and square root (-prec-div=false -prec-sqrt=false,
+about 2 ulp): their results are compared with the FP64 path through a
+tolerance.  That path's pressure recovery is made of explicitly rounded FP32
+operations on pairs of floats, which the flags leave alone (its reciprocal of
+the density is corrected for whichever division gave it); its face field stays
+FP64.
 The discrete adjoint (adjoint.cu) has no counterpart in the reference: its
 FP64 products and sums are fused (fewer instructions on the FP64 pipe, one
 rounding fewer each).

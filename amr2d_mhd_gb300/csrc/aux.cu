@@ -139,10 +139,10 @@ namespace {
 // The widest CTAs with which all leaves are resident at once, else 128 threads:
 // the 400 cells of a leaf take 1, 2 or 4 rounds.  KH meshes, us per step with
 // the cooperative launch / 128 / 224 / 416 threads: FP32 16 leaves 79 / - / 76 /
-// 72, 196: 90 / - / 86 / 82.5, 400: 134 / 111 / 104 / 100 (95.5 in a second run,
-// 224: 99.8), 576: - / 121 / 113 / 124, 784: - / 146 / 142 / 149, 1024: 215 / 168
-// / 175 / 179, 4096: 754 / 574 / 589 / 642; FP64 196: 236 / - / 232 / 230, 324:
-// 352 / 343 / 334 / 340, 576: - / 541 / 532 / 539, 784: - / 725 / 729 / 732.
+// 72, 196: 90 / - / 86 / 82.5, 400: 134 / 111 / 100 / 95.5, 576: - / 121 / 113 /
+// 124, 784: - / 146 / 142 / 149, 1024: 215 / 168 / 175 / 179, 4096: 754 / 574 / 589
+// / 642; FP64 196: 236 / - / 232 / 230, 324: 352 / 343 / 334 / 340, 576: - / 541 /
+// 532 / 539, 784: - / 725 / 729 / 732.
 int ct_threads(const Method &m, int n) {
   for (const int t : {416, 224})
     if (n <= sm_count() * (m.f32 ? ct_resident<float>(t) : ct_resident<double>(t))) return t;

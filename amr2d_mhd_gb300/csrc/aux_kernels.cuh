@@ -15,10 +15,9 @@ namespace amr {
 // (GhostLaunch and the gather of one op: ghost.cuh)
 
 // save the pre-fill values the same fill overwrites; the first CTA takes the
-// step's parameters from host memory.  (As copies of their own, the parameters
-// before the step's kernels, the two per-leaf results of k_dt_cell and the error
-// status after them took 7.5 us of each step: FP32 rotor of 196 leaves 114 us a
-// step with them, 106.6 without.)
+// step's parameters from host memory.  (FP32 rotor of 196 leaves: 106.6 us a step,
+// 114 with copies for the parameters, for k_dt_cell's two per-leaf results and for
+// the error record.)
 template <int N>
 __global__ void k_ghost_snap(GhostLaunch g) {
   pdl_wait();
@@ -223,8 +222,8 @@ __device__ __forceinline__ void ct_cell_block(const CtArgs &a, const FillFuse &f
 // rule at launch_ct_emf in aux.cu).  Few leaves wait for rounds of dependent
 // loads, so wide CTAs; many wait for the loads of their fills' gathers, so
 // registers are held to 40 (64 in FP64) for 1536 (1024) resident threads per SM.
-// 6272 FP32 leaves: EMF 121, faces 50, cells 40 us (121, 58, 52 before the
-// conversions and products left the FP64 pipe).
+// 6272 FP32 leaves: EMF 121, faces 50, cells 40 us (121, 58, 52 with conversions
+// and products on the FP64 pipe).
 template <typename S> __host__ __device__ constexpr int ct_resident(int threads) {
   return sizeof(S) == 4 ? (threads == 416 ? 3 : (threads == 224 ? 6 : 12)) : (threads == 416 ? 2 : (threads == 224 ? 4 : 8));
 }
@@ -345,11 +344,11 @@ __global__ void __launch_bounds__(128) k_diffuse(CtArgs a) {
 // NaN trap on every cell, as k_prim), then one thread per interior cell
 // forms the wave speeds and the criterion from them (FP64 for the FP64 path;
 // the FP32 path computes the cell values in FP32 and reduces them in FP64).
-// The FP64 form was bound by the FP64 pipe; with divisions, roots and the
-// criterion's maxima on the integer pipe (softfp.cuh) it takes 25 us for the
-// 196 leaves of a rotor, 60 before.  The FP32 form was bound by the FP64
-// instructions of the pressure recovery (76 % busy); with pairs of floats
-// (cons2prim_cell) 85 us for 6272 leaves, 103 before.
+// The FP64 form has its divisions, roots and the criterion's maxima on the
+// integer pipe (softfp.cuh): 25 us for the 196 leaves of a rotor, 60 with them on
+// the FP64 pipe.  The FP32 form recovers the pressure without that pipe
+// (cons2prim_cell): 85 us for 6272 leaves, 103 with FP64 sums, which kept it 76 %
+// busy.
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

@@ -136,7 +136,7 @@ class Engine {
   int upload_params();
   void fill_params_host();
   int enqueue_stage_sequence();
-  int enqueue_step();              // params upload, stage sequence, dt kernels, result copies
+  int enqueue_step();              // parameters, stage sequence, dt kernel
   int launch_step();               // launch_step_work, bracketed by events when profiling
   int launch_step_work();          // enqueue_step directly or as a replayed CUDA graph
   int fill(std::initializer_list<std::pair<FillKind, int>> what);

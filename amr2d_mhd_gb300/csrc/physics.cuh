@@ -261,7 +261,10 @@ __device__ __forceinline__ void fast_speeds(M &m, const T *w, T gamma, T *cf) {
   }
 }
 
-// FP32: as fast_speed_of, with one reciprocal for both
+// FP32: as fast_speed_of, with one reciprocal for both.  Error against 64 bits
+// over rotor, blast, low-beta and KH states: rms 3.8e-8, at most 1.9e-7 (the
+// form with the roots, each quotient correctly rounded: 4.8e-8 and 2.1e-6, as its
+// difference c_a^2 - c_n^2 cancels).
 __device__ __forceinline__ void fast_speeds_of(Native<float> &m, const float *w, float gamma, float *cf) {
   const float ir = 1.f / w[0];
   const float bx = w[5] * w[5] * ir, by = w[6] * w[6] * ir, bz = w[7] * w[7] * ir, a2 = gamma * w[4] * ir;

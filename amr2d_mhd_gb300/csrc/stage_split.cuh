@@ -163,10 +163,9 @@ __global__ void __launch_bounds__(128, MINB) k_faces_persist(const __grid_consta
 
 // persistent variant with dynamic work distribution: a grid of the CTAs the
 // SMs hold at once, each warp claiming the next 32 faces of the step's face
-// list from a global counter, so that warps that met cheap faces (uniform
-// regions, where the limiter ratios need no division) take more; the last
-// CTA to finish zeroes the counters for the next launch (every CTA has left
-// its loop by then, so nothing claims work any more)
+// list from a global counter, so that a warp that was quick takes more; the
+// last CTA to finish zeroes the counters for the next launch (every CTA has
+// left its loop by then, so nothing claims work any more)
 template <int NG, int RECON, int FLUX, typename S, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_faces_dyn(const __grid_constant__ SplitArgs a) {
   pdl_wait();

@@ -1,8 +1,9 @@
-"""The FP32 path's pressure recovery (cons2prim_cell<float> in
-amr2d_mhd_gb300/csrc/stage.cuh), restated with numpy on the CPU: the sums of
+"""The pairs of floats of the FP32 path's pressure recovery (cons2prim_cell<float>
+in amr2d_mhd_gb300/csrc/stage.cuh), restated with numpy on the CPU: the sums of
 squares and |m|^2/rho as FP32 hi + lo pairs (Dekker's exact product through
-an FMA, Knuth's TwoSum, the reciprocal corrected by its FMA residual), then
-E - (|m|^2/rho + |B|^2)/2 and gamma - 1 in FP64.  An FP32 FMA is emulated
+an FMA, Knuth's TwoSum, the reciprocal corrected by its FMA residual), here with
+E - (|m|^2/rho + |B|^2)/2 and gamma - 1 in FP64, the form whose error the library's
+sums of floats are measured against (tests/test_gpu_fp32_pressure.py runs those).  An FP32 FMA is emulated
 exactly: the product of two FP32 values is exact in FP64, and so is its sum
 with an FP32 value of the same magnitude, so one rounding to FP32 gives the
 FMA's result.  The test bounds the error of the recovered pressure against
@@ -34,7 +35,7 @@ def sum_sq3(a, b, c):
 
 
 def pressure_df(u, g):
-    """Mode 2 of cons2prim_cell<float> (the default)."""
+    """The pairs summed in FP64."""
     ir = F(F(1) / u[0])
     rl = F(fma32(-u[0], ir, F(1)) * ir)
     mh, ml = sum_sq3(u[1], u[2], u[3])

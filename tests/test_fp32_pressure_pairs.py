@@ -1,6 +1,7 @@
-"""The FP32 path's pressure recovery with pairs of floats throughout
-(cons2prim_cell<float> in amr2d_mhd_gb300/csrc/stage.cuh), restated with numpy
-on the CPU: its error against an exact rational evaluation, beside that of the
+"""The FP32 path's pressure recovery with pairs of floats throughout, restated with
+numpy on the CPU (cons2prim_cell<float> in amr2d_mhd_gb300/csrc/stage.cuh adds the
+low parts of its sums without rounding, tests/test_gpu_fp32_pressure.py; here they
+are rounded): its error against an exact rational evaluation, beside that of the
 same sums taken in FP64 and rounded to FP32 at the end.  The unrounded pair has
 to be good to 2^-43 of the subtracted terms (the bound of the form with FP64
 sums), and the FP32 result within one and a half units of the rounded FP64

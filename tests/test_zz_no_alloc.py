@@ -3,9 +3,9 @@
 Hosts that may not call cudaMalloc when they need the time step -- code
 inside a captured CUDA graph, allocator-free real-time loops, frameworks that
 own every device allocation -- call amr_cfl_dt_static with their own device
-arrays; its per-block scratch is a fixed 65536-entry array in the library's
-device globals.  The test checks it through the C ABI against amr_cfl_dt, on
-two calls in a row, with 2 ghost layers (MUSCL) and 4 (WENO5).  This file
+arrays; it has no scratch.  The test checks it through the C ABI against
+amr_cfl_dt, on two calls in a row, with 2 ghost layers (MUSCL) and 4 (WENO5);
+tests/test_gpu_cfl_static_edges.py has the edges of the reduction.  This file
 sorts last so that a run that stops at the first failure has already run
 every other test.
 """
